@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "../../include/nhflood.h"
+#include "nhf_math.cuh"
 
 namespace nhf {
 
@@ -182,6 +183,44 @@ __device__ __forceinline__ real cfl_value(real afa, real g, real length, real q,
 {
     return afa * length / (sqrt(g * h) + fabs(q) / h);
 }
+
+#ifndef NHF_REAL_DOUBLE
+// Two tests that spare a step its exact quotients and square roots where they
+// cannot matter. Both use the hardware's approximate reciprocal and root
+// (relative error at most 2^-22 each) with a margin of 2^-16, so a value they
+// rule out is out by more than all roundings together; a NaN rules out nothing.
+
+// The CFL value `scale` / (sqrt(g h) + |q| / h) of a side (scale = afa L, h >=
+// 0.01) is certainly above `best`: the exact value need not be formed.
+__device__ __forceinline__ bool cfl_above(float scale, float g, float q, float h, float best)
+{
+    const float below = approx_sqrt(g * h) + fabsf(q) * approx_rcp(h);
+    return scale > best * below * (1.0f + 0x1p-16f);
+}
+
+// The speed of a wet cell of depth h (>= 0.01) with face sums qx = ql + qr and
+// qy = qb + qt is certainly not above `fastest`, its maximum so far.
+__device__ __forceinline__ bool speed_not_above(float qx, float qy, float height, float width, float h, float fastest)
+{
+    const float r = 0.5f * approx_rcp(h);
+    const float u = qx * approx_rcp(height) * r, v = qy * approx_rcp(width) * r;
+    return (u * u + v * v) * (1.0f + 0x1p-16f) + 0x1p-120f < fastest * fabsf(fastest);
+}
+
+// The running maximum of a cell's speed (solver_compact.py:355-362, 580-590):
+// `fastest`, or the exact speed where it is above it (a dry cell's is zero).
+__device__ __forceinline__ float fastest_speed(bool wet, float qx, float qy, float height, float width, float h,
+                                               float fastest)
+{
+    if (wet ? speed_not_above(qx, qy, height, width, h, fastest) : !(fastest < 0.0f)) return fastest;
+    // x / 2 and x * 0.5 are the same correctly rounded value
+    const float u = wet ? qx / height / h * 0.5f : 0.0f;
+    const float v = wet ? qy / width / h * 0.5f : 0.0f;
+    const float s2 = u * u + v * v;
+    const float speed = s2 == 0.0f ? 0.0f : sqrtf(s2);
+    return speed > fastest ? speed : fastest;
+}
+#endif
 
 // flow_depth_t[si] (solver_compact.py:628-630) from a depth array; side 0
 // keeps the field's initial zero.

@@ -165,15 +165,9 @@ __device__ __forceinline__ real lattice_update(const Dev &d, const LatticePlan &
     raw_depth -= removed;
     real floor_v = rmax(-raw_depth, RC(0));
     real depth = kind == 0 ? rmax(d.level_values[bi] - z, RC(0)) : rmax(raw_depth, RC(0));
-    real h = rmax(depth, RC(0.01));
-    real u = RC(0), v = RC(0);
-    if (depth >= d.min_h) {
-        u = (ql + qr) / P.height / h * RC(0.5);
-        v = (qb + qt) / P.width / h * RC(0.5);
-    }
-    real s2 = u * u + v * v;
-    real speed = s2 == RC(0) ? RC(0) : sqrt(s2);
-    if (speed > k.max_speed) P.max_speed[L] = speed;
+    const real fastest = fastest_speed(depth >= d.min_h, ql + qr, qb + qt, P.height, P.width, rmax(depth, RC(0.01)),
+                                       k.max_speed);
+    if (fastest > k.max_speed) P.max_speed[L] = fastest;
     if (depth > k.max_depth) {
         P.max_depth[L] = depth;
         P.peak_hi[L] = __ldg(step_end);  // the clock words are not written during the march
@@ -211,12 +205,14 @@ __device__ __forceinline__ real lattice_update(const Dev &d, const LatticePlan &
 }
 
 // CFL candidate (solver_compact.py:617-641) of one interior side, folded
-// into the running minimum key (dt bits << 32 | side id); the side id is
-// read only for a candidate at or below the minimum.
+// into the running minimum key (dt bits << 32 | side id); only a candidate
+// that may be at or below the minimum is formed exactly, and only then is the
+// side id read.
 __device__ __forceinline__ void lattice_cfl(const Dev &d, real len, real q, real za, real ha, real zb, real hb,
                                             const int32_t *side_ids, size_t L, unsigned long long &best)
 {
     const real fd = cfl_face_depth(za, ha, zb, hb);
+    if (cfl_above(d.afa * len, d.g, q, fd, __uint_as_float((uint32_t)(best >> 32)))) return;
     const uint32_t bits = __float_as_uint(cfl_value(d.afa, d.g, len, q, fd));
     if (bits <= (uint32_t)(best >> 32)) {
         const unsigned long long key = ((unsigned long long)bits << 32) | (unsigned)__ldg(side_ids + L);

@@ -8,6 +8,10 @@
 // result does not depend on a vendor math library and is reproduced bit for
 // bit by the CPU restatement used in the tests. Build with --fmad=false.
 //
+// The F32 step takes friction_pow and horton_exp below: shorter evaluations of
+// the same two values that give the same F32 bits (Ziv's rounding test, the
+// full evaluation where the short one cannot decide the rounding).
+//
 // Methods (published):
 //  ln  : x = m * 2^e, m in [sqrt(1/2), sqrt(2)]; ln m = 2 atanh(s) with
 //        s = (m - 1) / (m + 1) and the odd Taylor series of atanh to s^25;
@@ -93,8 +97,99 @@ __device__ __forceinline__ float pow_f32(float x, float y)
 
 __device__ __forceinline__ float exp_f32(float a) { return (float)exp_f64((double)a); }
 
-// The same two functions in the build's physics type: rounded once to F32,
-// or in the FP64 build kept in double.
+__device__ __forceinline__ float approx_lg2(float x)
+{
+    float r;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float approx_ex2(float x)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float approx_rcp(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float approx_sqrt(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// Whether an FP64 value lies so near the midpoint of two F32 neighbours (4096
+// FP64 units, at least 2^-41 of the value) that a relative error of 2^-41
+// could change its rounding to F32.
+__device__ __forceinline__ bool rounding_open(double v)
+{
+    const uint32_t below = (uint32_t)__double_as_longlong(v) & 0x1fffffffu;  // the 29 bits F32 drops
+    return below - (0x10000000u - 4096u) < 8192u;
+}
+
+// The full evaluations behind the rounding test, out of line: about one in
+// 2^16 arguments gets here.
+static __device__ __noinline__ float pow73_full(float x) { return pow_f32(x, 0x1.2aaaaap+1f); }
+static __device__ __noinline__ float exp_full(float a) { return exp_f32(a); }
+
+// x ** f32(7/3) for the friction factor, x >= 1e-5: the value of
+// pow_f32(x, 7/3). With the F32 exponent y = 7/3 - c (c = 7.947e-8),
+// x^y = x^3 (x^(-1/3))^2 x^(-c). x^(-1/3) is an F32 estimate s (relative
+// error below 2^-18) corrected by the binomial series of (1 - t)^(-1/3) at
+// t = 1 - x s^3, whose third term is under 2^-50; x^(-c) is 1 + w + w^2 / 2 at
+// w = -c ln x, |w| < 2e-6, in F32 (error under 2^-43). 11 FP64 operations
+// instead of about 85, and a shorter chain, which is what a small step's
+// momentum waits for. Measured together with horton_exp, cfl_above and
+// speed_not_above (nhf_common.cuh), 32 steps: 256 x 256 cells 732 to 682 us,
+// 2048 x 1531 cells with Horton soil 9.34 to 7.95 ms, quadtree of 1.36 M cells
+// 5.98 to 5.36 ms.
+__device__ __forceinline__ float friction_pow(float x)
+{
+    const float lg = approx_lg2(x);
+    const double xd = (double)x, s = (double)approx_ex2(lg * -0x1.555556p-2f);
+    const double t = __fma_rn(-xd, s * s * s, 1.0);
+    const double r = __fma_rn(s * t, __fma_rn(t, 2.0 / 9.0, 1.0 / 3.0), s);
+    const double a = xd * r;
+    const double v = (xd * xd) * (a * r);
+    const float w = lg * (float)(-(7.0 / 3.0 - 0x1.2aaaaap+1) * 0.693147180559945309);
+    const double p = __fma_rn(v, (double)fmaf(0.5f * w, w, w), v);
+    if (rounding_open(p) || !(x < 0x1p20f)) return pow73_full(x);
+    return (float)p;
+}
+
+// exp(a) of the Horton capacity, a <= 0: the value of exp_f32(a). One-step
+// reduction by ln 2 (|a| < 80: error under 2^-46) and the Taylor series to
+// degree 10 (remainder under 2^-41.9 for |r| <= ln2 / 2) with fused
+// multiply-adds: 14 FP64 operations instead of about 40.
+__device__ __forceinline__ float horton_exp(float a)
+{
+    const float n = rintf(a * 0x1.715476p+0f);
+    const double r = __fma_rn((double)n, -0x1.62e42fefa39efp-1, (double)a);
+    double p = 1.0 / 3628800.0;
+    p = __fma_rn(p, r, 1.0 / 362880.0);
+    p = __fma_rn(p, r, 1.0 / 40320.0);
+    p = __fma_rn(p, r, 1.0 / 5040.0);
+    p = __fma_rn(p, r, 1.0 / 720.0);
+    p = __fma_rn(p, r, 1.0 / 120.0);
+    p = __fma_rn(p, r, 1.0 / 24.0);
+    p = __fma_rn(p, r, 1.0 / 6.0);
+    p = __fma_rn(p, r, 0.5);
+    p = __fma_rn(p, r, 1.0);
+    p = __fma_rn(p, r, 1.0);
+    p *= __longlong_as_double((long long)((int)n + 1023) << 52);
+    if (rounding_open(p) || !(a > -80.0f && a <= 0.0f)) return exp_full(a);
+    return (float)p;
+}
+
+// The friction power and the Horton exponential in the build's physics type:
+// rounded once to F32, or in the FP64 build kept in double.
 #ifdef NHF_REAL_DOUBLE
 __device__ __forceinline__ double pow_real(double x, double y)
 {
@@ -104,8 +199,9 @@ __device__ __forceinline__ double pow_real(double x, double y)
 }
 __device__ __forceinline__ double exp_real(double a) { return exp_f64(a); }
 #else
-__device__ __forceinline__ float pow_real(float x, float y) { return pow_f32(x, y); }
-__device__ __forceinline__ float exp_real(float a) { return exp_f32(a); }
+// (the F32 step's exponent is f32(7/3) throughout)
+__device__ __forceinline__ float pow_real(float x, float) { return friction_pow(x); }
+__device__ __forceinline__ float exp_real(float a) { return horton_exp(a); }
 #endif
 
 }  // namespace nhf

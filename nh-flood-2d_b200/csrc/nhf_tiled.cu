@@ -140,6 +140,17 @@ __device__ __forceinline__ float term_value(int t, int B, float removed, float f
     return (t - 4 - 5 * B == bi) ? discharge : 0.0f;
 }
 
+// CFL candidate (solver_compact.py:628-631) of an interior side with face depth
+// h, folded into the running minimum key (dt bits << 32 | side id); the exact
+// value is formed only where it may be at or below the minimum.
+__device__ __forceinline__ void fold_cfl(const Dev &d, float len, float q, float h, unsigned gid,
+                                         unsigned long long &best)
+{
+    if (cfl_above(d.afa * len, d.g, q, h, __uint_as_float((uint32_t)(best >> 32)))) return;
+    const unsigned long long key = ((unsigned long long)__float_as_uint(cfl_value(d.afa, d.g, len, q, h)) << 32) | gid;
+    best = key < best ? key : best;
+}
+
 // One fused step of tile t of the mesh described by d (n_tiles tiles).
 // kHang: 0 no hanging edges, 1 hanging edges, 2 decided by d at run time.
 // kGate (256-cell tiles, separate CFL pass): the gate controller's source
@@ -293,7 +304,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             }
             float xdq = (d.neg_g * difference / dx) * maxf(xwh, 0.0f) * dt;
             float ratio = 0.0f;
-            if (xq != 0.0f) ratio = xq / pow_f32(maxf(xwh, 0.00001f), d.seven_thirds);
+            if (xq != 0.0f) ratio = xq / pow_real(maxf(xwh, 0.00001f), d.seven_thirds);
             float xf = 1.0f + d.g * dt * (n * n) * fabsf(ratio);
             float nb;
             if (kThetaOne) {
@@ -443,7 +454,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             rt_out[g] = rt;
             float f0 = in_f0[kk], fc = in_fc[kk];
             float diff = f0 - fc;
-            infil = diff == 0.0f ? fc + 0.0f : fc + diff * exp_f32(-in_k[kk] * rt / 3600.0f);
+            infil = diff == 0.0f ? fc + 0.0f : fc + diff * exp_real(-in_k[kk] * rt / 3600.0f);
             if (__float_as_uint(infil) != __float_as_uint(in_inf[kk])) m.infiltration[g] = infil;
         } else {
             infil = in_inf[kk];
@@ -478,16 +489,9 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         }
         depth_out[g] = depth;
         sh_s[slot] = depth;
-        float h = maxf(depth, 0.01f);
-        float u = 0.0f, v = 0.0f;
-        if (depth >= d.min_h) {
-            // x / 2 and x * 0.5 are the same correctly rounded value
-            u = (ql + qr) / in_hgt[kk] / h * 0.5f;
-            v = (qb + qt) / in_wid[kk] / h * 0.5f;
-        }
-        float s2 = u * u + v * v;
-        float speed = s2 == 0.0f ? 0.0f : sqrtf(s2);
-        if (speed > in_ms[kk]) m.max_speed[g] = speed;
+        const float fastest = fastest_speed(depth >= d.min_h, ql + qr, qb + qt, in_hgt[kk], in_wid[kk],
+                                            maxf(depth, 0.01f), in_ms[kk]);
+        if (fastest > in_ms[kk]) m.max_speed[g] = fastest;
         if (depth > in_md[kk]) {
             m.max_depth[g] = depth;
             m.peak_hi[g] = step_hi; m.peak_lo[g] = step_lo;
@@ -545,7 +549,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             float rt = rt_in[g] + dt;
             float f0 = m.f0[g], fc = m.fc[g];
             float diff = f0 - fc;
-            infil = diff == 0.0f ? fc + 0.0f : fc + diff * exp_f32(-m.k[g] * rt / 3600.0f);
+            infil = diff == 0.0f ? fc + 0.0f : fc + diff * exp_real(-m.k[g] * rt / 3600.0f);
         } else {
             infil = m.infiltration[g];
         }
@@ -658,9 +662,6 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     // owned sides with the new depths (the split form's CFL pass follows).
     const bool split = P.split != 0;
     unsigned long long best = kCflEmpty;
-    // A side at the 0.01 m face-depth floor with q = 0 has the CFL value
-    // afa * L / sqrt(g * 0.01); it is reused while L repeats.
-    float dry_len = -1.0f, dry_cfl = 0.0f;
     for (int j = tid; j < tl.n_owned; j += NT) {
         const int gid = tl.sbase + tl.srel[j];
         float qv = sh_q[j];
@@ -672,18 +673,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             float zl = sh_z[a], zh = sh_z[b];
             float head = maxf(zl + sh_s[a], zh + sh_s[b]);
             float h = maxf(head - maxf(maxf(zl, zh), kDh), 0.01f);
-            float cfl;
-            if (h == 0.01f && qv == 0.0f) {
-                if (sh_len[j] != dry_len) {
-                    dry_len = sh_len[j];
-                    dry_cfl = d.afa * dry_len / (sqrtf(d.g * h) + fabsf(qv) / h);
-                }
-                cfl = dry_cfl;
-            } else {
-                cfl = d.afa * sh_len[j] / (sqrtf(d.g * h) + fabsf(qv) / h);
-            }
-            unsigned long long key = ((unsigned long long)__float_as_uint(cfl) << 32) | (unsigned)gid;
-            best = key < best ? key : best;
+            fold_cfl(d, sh_len[j], qv, h, (unsigned)gid, best);
         }
     }
     if (!split) {
@@ -753,9 +743,7 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
                 const float zl = m.bed[el], zh = m.bed[eh];
                 const float head = maxf(zl + depth[el], zh + depth[eh]);
                 const float h = maxf(head - maxf(maxf(zl, zh), kDh), 0.01f);
-                const float cfl = d.afa * m.length[si] / (sqrtf(d.g * h) + fabsf(q[si]) / h);
-                const unsigned long long key = ((unsigned long long)__float_as_uint(cfl) << 32) | (unsigned)si;
-                best = key < best ? key : best;
+                fold_cfl(d, m.length[si], q[si], h, (unsigned)si, best);
             }
         }
     }
