@@ -94,55 +94,45 @@ __global__ void k_prepare(Dev d)
 
 // ------------------------------------------------------ pressure (pressure.py)
 
-__device__ void face_difference(const Dev &d, const real *depth, int cell, int direction, int axis,
-                                real &value_out, real &distance_out, int &usable_out)
+// The hanging-edge gradients' inputs from the mesh tables, once per solve; a
+// thread per (cell, axis). Sums run in the order hang_face takes them.
+__global__ void k_hang_setup(Dev d)
 {
     const nhf_mesh &m = d.m;
-    real value = RC(0.0), distance = RC(0.0), total = RC(0.0);
-    int usable = 1;
-    real eta = m.bed[cell] + depth[cell];
-    int start = m.face_ptr[4 * cell + direction];
-    int count = m.face_count[4 * cell + direction];
-    for (int j = 0; j < count; ++j) {
-        int side = m.isl_data[start + j];
-        int other = m.topology[3 * side + 1] + m.topology[3 * side + 2] - cell;
-        if (other == 0 || depth[other] <= d.min_h) {
-            usable = 0;
-        } else {
-            real weight = m.length[side];
-            value += weight * ((m.bed[other] + depth[other]) - eta);
-            real delta = axis == 1 ? m.y[other] - m.y[cell] : m.x[other] - m.x[cell];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * m.hang_cells) return;
+    const int cell = m.hcells[i >> 1], axis = i & 1;
+    HangItem it{};
+    it.cell = m.axes[i] == 1 ? cell : -1;
+    for (int f = 0; f < 2; ++f) {
+        const int start = m.face_ptr[4 * cell + 2 * axis + f], count = m.face_count[4 * cell + 2 * axis + f];
+        it.other[f][0] = it.other[f][1] = -1;
+        real total = RC(0), distance = RC(0);
+        bool open = count > 0;
+        for (int j = 0; j < count && j < 2; ++j) {
+            const int side = m.isl_data[start + j];
+            const int other = m.topology[3 * side + 1] + m.topology[3 * side + 2] - cell;
+            const real weight = m.length[side];
+            const real delta = axis == 1 ? m.y[other] - m.y[cell] : m.x[other] - m.x[cell];
             distance += weight * delta;
             total += weight;
+            open = open && other != 0;
+            it.other[f][j] = other;
+            it.weight[f][j] = weight;
         }
+        if (count > 2 && it.cell >= 0) it.cell = -2;
+        if (!open || !(total > RC(0))) it.other[f][0] = it.other[f][1] = -1;
+        it.total[f] = total;
+        it.reach[f] = distance / total;
     }
-    if (total > RC(0.0)) { value /= total; distance /= total; }
-    else usable = 0;
-    value_out = value; distance_out = distance; usable_out = usable;
+    d.hang[i] = it;
 }
 
 __global__ void k_pressure(Dev d)
 {
-    const nhf_mesh &m = d.m;
     if (!d.ctl->active) return;
     int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= m.hang_cells) return;
-    int cell = m.hcells[slot];
-    const real *depth = cur_depth(d, d.ctl->parity);
-    for (int axis = 0; axis < 2; ++axis) {
-        if (m.axes[2 * slot + axis] != 1) continue;
-        real value = RC(0.0);
-        if (depth[cell] > d.min_h) {
-            int minus = axis == 1 ? 2 : 0, plus = axis == 1 ? 3 : 1;
-            real dm, xm, dp, xp; int okm, okp;
-            face_difference(d, depth, cell, minus, axis, dm, xm, okm);
-            face_difference(d, depth, cell, plus, axis, dp, xp, okp);
-            if (okm && okp) value = (dp - dm) / (xp - xm);
-            else if (okm) value = dm / xm;
-            else if (okp) value = dp / xp;
-        }
-        d.gradients[2 * slot + axis] = value;
-    }
+    if (slot < d.m.hang_cells) hang_slot(d, slot);
 }
 
 // ----------------------------------------------------------- theta < 1 faces
@@ -1045,6 +1035,7 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     size_t o_fqn = take(theta_one ? 32 : sizeof(real) * 4 * (size_t)e);
     size_t o_eq = take(sizeof(real) * 4 * (size_t)e);
     size_t o_grad = take(sizeof(real) * 2 * hc);
+    size_t o_hang = take(sizeof(HangItem) * 2 * hc);
     size_t o_accs = take(sizeof(double) * (size_t)blocks * T);
     size_t o_accc = take(sizeof(double) * (size_t)blocks * T);
     size_t o_begin = take(sizeof(real) * 4);  // also the staging of nhf_get_cfl's three words
@@ -1085,6 +1076,7 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     d.face_qn = (real *)(base + o_fqn);
     d.eq = (real *)(base + o_eq);
     d.gradients = (real *)(base + o_grad);
+    d.hang = (HangItem *)(base + o_hang);
     d.acc_sum = (double *)(base + o_accs);
     d.acc_comp = (double *)(base + o_accc);
     if (h->tiled) {
@@ -1141,6 +1133,7 @@ int nhf_initialize(nhf_handle *h)
     int rc = enter(h); if (rc) return rc;
     int n = h->m.e_num > h->m.s_num ? h->m.e_num : h->m.s_num;
     k_initialize<<<grid_for(n, 256), 256, 0, h->s>>>(h->dev);
+    if (h->m.hang_cells > 0) k_hang_setup<<<grid_for(2 * h->m.hang_cells, 256), 256, 0, h->s>>>(h->dev);
     return leave(h);
 }
 

@@ -1179,53 +1179,11 @@ void launch_step(const Dev &d, size_t smem, cudaStream_t s)
 
 // Tangential gradients for the tiled form (reads the current-parity depth).
 namespace {
-__device__ __forceinline__ void pressure_slot(const Dev &d, int slot)
-{
-    const nhf_mesh &m = d.m;
-    const float *depth = cur_depth(d, d.ctl->parity);
-    int cell = m.hcells[slot];
-    for (int axis = 0; axis < 2; ++axis) {
-        if (m.axes[2 * slot + axis] != 1) continue;
-        float value = 0.0f;
-        if (depth[cell] > d.min_h) {
-            float dv[2], xv[2];
-            int ok[2];
-            for (int side_of = 0; side_of < 2; ++side_of) {
-                int direction = axis == 1 ? 2 + side_of : side_of;
-                float val = 0.0f, distance = 0.0f, total = 0.0f;
-                int usable = 1;
-                float eta = m.bed[cell] + depth[cell];
-                int start = m.face_ptr[4 * cell + direction], count = m.face_count[4 * cell + direction];
-                for (int j = 0; j < count; ++j) {
-                    int side = m.isl_data[start + j];
-                    int other = m.topology[3 * side + 1] + m.topology[3 * side + 2] - cell;
-                    if (other == 0 || depth[other] <= d.min_h) {
-                        usable = 0;
-                    } else {
-                        float weight = m.length[side];
-                        val += weight * ((m.bed[other] + depth[other]) - eta);
-                        float delta = axis == 1 ? m.y[other] - m.y[cell] : m.x[other] - m.x[cell];
-                        distance += weight * delta;
-                        total += weight;
-                    }
-                }
-                if (total > 0.0f) { val /= total; distance /= total; }
-                else usable = 0;
-                dv[side_of] = val; xv[side_of] = distance; ok[side_of] = usable;
-            }
-            if (ok[0] && ok[1]) value = (dv[1] - dv[0]) / (xv[1] - xv[0]);
-            else if (ok[0]) value = dv[0] / xv[0];
-            else if (ok[1]) value = dv[1] / xv[1];
-        }
-        d.gradients[2 * slot + axis] = value;
-    }
-}
-
 __global__ void k_pressure_tiled(const __grid_constant__ Dev d)
 {
     if (!d.ctl->active) return;
     int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot < d.m.hang_cells) pressure_slot(d, slot);
+    if (slot < d.m.hang_cells) hang_slot(d, slot);
 }
 
 // length-weighted face discharge for theta < 1 (solver_compact.py:118-132)
@@ -1292,7 +1250,7 @@ __global__ void k_ens_pressure(const Dev *devs, const int2 *items)
     const Dev &d = devs[w.x];
     if (!d.ctl->active) return;
     const int end = min(d.m.hang_cells, (w.y + 1) * kEnsChunk);
-    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x) pressure_slot(d, i);
+    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x) hang_slot(d, i);
 }
 
 __global__ void k_ens_face_qn(const Dev *devs, const int2 *items)
@@ -1473,7 +1431,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
 void tiled_enqueue_step(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate)
 {
     const nhf_mesh &m = d.m;
-    if (m.hang_cells > 0) k_pressure_tiled<<<(m.hang_cells + 255) / 256, 256, 0, s>>>(d);
+    if (m.hang_cells > 0) k_pressure_tiled<<<(m.hang_cells + 63) / 64, 64, 0, s>>>(d);
     if (!d.theta_one) k_face_qn_tiled<<<(m.e_num + 255) / 256, 256, 0, s>>>(d);
     if (gate) {  // 256-cell tiles, split plan (checked when the controller is attached)
         const int grid = d.plan.n_tiles;

@@ -40,7 +40,7 @@ def device_bytes_estimate(arrays) -> int:
     plan)."""
     e, s = arrays.e_num, arrays.s_num
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * arrays.terms
+    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * arrays.terms + 128 * arrays.hang_cells
     plan = 24 * e + 64 * 1024
     return int(arrays.nbytes() + state + scratch + plan + (1 << 20))
 
@@ -48,13 +48,15 @@ def device_bytes_estimate(arrays) -> int:
 def device_bytes_bound(workload) -> int:
     """An upper bound of device_bytes_estimate from the mesh sizes alone
     (before the step arrays are built): hanging-edge tables counted as if
-    every side had one."""
+    every side had one, gradient cells as all the cells at faces of several
+    sides."""
     m = workload.mesh
     e, s, isl = m.e_num, m.s_num, len(m.isl_data)
+    hanging = min(e, 2 * int(m.counts[m.counts > 1].sum()))
     terms = 4 + 6 * len(workload.forcing.boundaries)
     inputs = 4 * (12 * e + 8 * e + isl) + 21 * s + 16 * e + 44 * s
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * terms
+    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * terms + 128 * hanging
     return int(inputs + state + scratch + 24 * e + 64 * 1024 + (1 << 20))
 
 
