@@ -92,6 +92,8 @@ def launches_per_batch(run) -> int:
     eng = run.engine
     if eng.path.startswith('lattice'):  # gather, begin, scatter, velocity; per step the step and its CFL pass
         return 4 + run.params.batch_size * 2
+    if 'resident=' in eng.path:  # the whole batch in one launch
+        return 1
     tiled = eng.path.startswith('tiled')
     pre = (1 if run.arrays.hang_cells else 0) + (0 if run.w.sita == 1.0 else 1)
     gate = run.arrays.gate

@@ -53,6 +53,9 @@ extern "C" {
 #define NHF_STEP_BAD_CFL 2
 #define NHF_STEP_BAD_DT 3
 #define NHF_STEP_OVERSHOOT 4
+/* Not a clock status: the blocks of a resident batch lost one another (a
+ * wait ran out); the batch's results are void and so are later ones. */
+#define NHF_STEP_STALLED 5
 
 /* The physics type of the build. The step computes in F32 as the
  * reference's fields do (libnhflood.so). Compiled with -DNHF_REAL_DOUBLE, the
@@ -108,9 +111,12 @@ typedef struct nhf_params {
     float min_dt;     /* F32(1e-4) CFL floor (solver_compact.py:31) */
     int32_t batch_size; /* steps per batch, 1..64 (clock.py:48-51) */
     int32_t path;       /* 0: the lattice form on a uniform grid it covers
-                           of at least 2^20 cells, else the fused tiled step
-                           when the mesh allows it,
-                           else multi-pass; 1: always the multi-pass step;
+                           of at least 2^20 cells, else the resident form
+                           (the whole batch in one cooperative launch) when
+                           one tile per SM covers the mesh, else the fused
+                           tiled step when the mesh allows it, else
+                           multi-pass; 4: the same without the resident form
+                           (members of an ensemble, which run beside others); 1: always the multi-pass step;
                            2: the lattice form when the mesh allows it, else
                            multi-pass; 3: the fused tiled step (tile size by
                            mesh size) when the mesh allows it, else multi-pass;

@@ -48,6 +48,8 @@ struct Ctl {
     uint32_t trace[NHF_MAX_BATCH * NHF_TRACE_COLS];
     unsigned long long cfl_min_bits;  // FP64 build: the CFL minimum's bits, then
     int32_t cfl_arg_min;              // the lowest side id that attains it
+    uint32_t epoch, batches;          // resident form: steps and batches so far
+    int32_t stalled;                  // resident form: a wait ran out
 };
 
 // Tile plan of the fused step (built on the host by nhf_tiled.cu).
@@ -62,6 +64,23 @@ struct TilePlan {
     const uint32_t *side_lohi; // local slots: lower | higher << 16
     const uint32_t *face_desc; // per slot 0..n_r012: start | counts (4 x 4 bits) << 16
     const uint16_t *face_idx;  // local side indices in the reference's CSR order
+};
+
+// What the resident form (nhf_resident.cu) adds to a tile plan of three rings:
+// its largest lists, the words blocks exchange and a batch's counters.
+struct ResidentArgs {
+    TilePlan plan;
+    int32_t max_don, max_hang, max_r1, max_owned;  // donor cells, hanging sides, ring-1 cells, owned sides of a tile
+    int32_t max_per_face;       // sides of a face
+    uint32_t words[4];          // the batch's target and origin ticks
+    // two buffers each, by the parity of the step
+    unsigned long long *keys;         // [2][tiles] phase bit, CFL bits, side id
+    unsigned long long *depth_words;  // [2][e_num] step, depth
+    unsigned long long *side_words;   // [2][s_num] step, final discharge
+    unsigned long long *face_words;   // [2][e_num][4] step, face discharge (theta < 1)
+    uint32_t *counts;                 // [2][steps][4] limited cells, limited faces, wet cells, min scale bits
+    int32_t *need_cell;               // [e_num] 1 depth, 2 face discharges are staged by another tile
+    uint8_t *need_side;               // [s_num] the discharge is staged by another tile
 };
 
 // Lattice form (nhf_lattice.cu) of a uniform mesh: the cells renumbered into
@@ -151,6 +170,14 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
     return v;
 }
 
+// The smallest of a warp's keys, in every lane.
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long v)
+{
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32));
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0xffffffffu);
+    return ((unsigned long long)hi << 32) | lo;
+}
+
 // Canonical pairwise tree over the 256 cells of one budget block:
 // slot i += slot i + stride for stride 128 .. 1. Returns the sum in thread 0.
 // Must be called by all 256 threads of the block.
@@ -210,6 +237,14 @@ __device__ __forceinline__ bool cfl_above(float scale, float g, float q, float h
     return scale > best * below * (1.0f + 0x1p-16f);
 }
 
+// The CFL value to within 2^-18; of two sides, one whose near value is above
+// kCflMargin times the other's is above it exactly.
+constexpr float kCflMargin = 1.0f + 0x1p-16f;
+__device__ __forceinline__ float cfl_near(float scale, float g, float q, float h)
+{
+    return scale * approx_rcp(approx_sqrt(g * h) + fabsf(q) * approx_rcp(h));
+}
+
 // The speed of a wet cell of depth h (>= 0.01) with face sums qx = ql + qr and
 // qy = qb + qt is certainly not above `fastest`, its maximum so far.
 __device__ __forceinline__ bool speed_not_above(float qx, float qy, float height, float width, float h, float fastest)
@@ -245,15 +280,16 @@ __device__ __forceinline__ real flow_depth_of(const nhf_mesh &m, const real *dep
     return rmax(head - rmax(rmax(zl, zh), kDh), RC(0.01));
 }
 
-// StepClock.choose (clock.py:94-167)
-__device__ __forceinline__ void clock_choose(const Dev &d, Ctl *c, float candidate, int slot)
+// StepClock.choose (clock.py:94-167) on a control block's clock; the trace row
+// takes the candidate, the event flag and a stop's status.
+template <class C>
+__device__ __forceinline__ void clock_choose(float min_dt, C *c, float candidate, uint32_t *row)
 {
-    uint32_t *row = c->trace + slot * NHF_TRACE_COLS;
     c->active = 0; c->dt = 0.0f; c->local = 0.0f; c->end_local = 0.0f;
     uint32_t now_hi = c->now[0], now_lo = c->now[1];
     uint32_t target_hi = c->next[0], target_lo = c->next[1];
     if (!(now_hi < target_hi || (now_hi == target_hi && now_lo < target_lo))) return;
-    if (!(candidate >= d.min_dt)) { row[3] = NHF_STEP_BAD_CFL; return; }
+    if (!(candidate >= min_dt)) { row[3] = NHF_STEP_BAD_CFL; return; }
     uint32_t borrow = now_lo > target_lo ? 1u : 0u;
     uint32_t rem_hi = target_hi - now_hi - borrow;
     uint32_t rem_lo = target_lo - now_lo;
@@ -311,7 +347,7 @@ __device__ __forceinline__ void clock_choose(const Dev &d, Ctl *c, float candida
 __device__ __forceinline__ void prepare_step(const Dev &d, Ctl *c, const real *depth, const real *q)
 {
     const nhf_mesh &m = d.m;
-    clock_choose(d, c, (float)c->ndt, c->slot);
+    clock_choose(d.min_dt, c, (float)c->ndt, c->trace + c->slot * NHF_TRACE_COLS);
     if (!c->active) return;
     c->limited_cells = 0; c->limited_faces = 0;
     c->min_scale_bits = real_bits(RC(1.0));
@@ -377,6 +413,34 @@ static __device__ __noinline__ bool hang_face(const Dev &d, const real *depth, i
     return usable;
 }
 
+__device__ __forceinline__ real hang_slope(const real dv[2], const real xv[2], const bool ok[2])
+{
+    if (ok[0] && ok[1]) return (dv[1] - dv[0]) / (xv[1] - xv[0]);
+    if (ok[0]) return dv[0] / xv[0];
+    if (ok[1]) return dv[1] / xv[1];
+    return RC(0);
+}
+
+// The gradient of a laid-out item from the depth and bed of its cell (dc, zc)
+// and of the cells across its faces.
+__device__ __forceinline__ real hang_from(const HangItem &it, real dc, real zc, const real ha[2][2],
+                                          const real za[2][2], real min_h)
+{
+    if (!(dc > min_h)) return RC(0);
+    const real eta = zc + dc;
+    real dv[2];
+    bool ok[2];
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+        const bool two = it.other[f][1] >= 0;
+        ok[f] = it.other[f][0] >= 0 && !(ha[f][0] <= min_h) && !(two && ha[f][1] <= min_h);
+        real val = RC(0) + it.weight[f][0] * ((za[f][0] + ha[f][0]) - eta);
+        if (two) val += it.weight[f][1] * ((za[f][1] + ha[f][1]) - eta);
+        dv[f] = val / it.total[f];
+    }
+    return hang_slope(dv, it.reach, ok);
+}
+
 // Tangential gradient of one (hanging cell, axis) on the given depths
 // (PressureReconstruction.update, pressure.py:65-115); 0 where it has none.
 // The item gives every address at once, so a gradient costs two memory
@@ -387,39 +451,26 @@ __device__ __forceinline__ real hang_gradient(const Dev &d, const real *depth, i
 {
     const nhf_mesh &m = d.m;
     const HangItem it = d.hang[2 * slot + axis];
-    const int cell = it.cell == -2 ? m.hcells[slot] : it.cell;
-    if (cell < 0) return RC(0);
-    real dv[2] = {RC(0), RC(0)}, xv[2] = {RC(1), RC(1)};
-    bool ok[2];
-    const real dc = depth[cell], eta = m.bed[cell] + dc;
+    if (it.cell == -1) return RC(0);
     if (it.cell == -2) {
+        const int cell = m.hcells[slot];
+        const real dc = depth[cell], eta = m.bed[cell] + dc;
+        real dv[2], xv[2];
+        bool ok[2];
         if (!(dc > d.min_h)) return RC(0);
         for (int f = 0; f < 2; ++f) ok[f] = hang_face(d, depth, cell, 2 * axis + f, axis, eta, dv + f, xv + f);
-    } else {
-        real ha[2][2], za[2][2];
-#pragma unroll
-        for (int f = 0; f < 2; ++f)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int o = it.other[f][j] < 0 ? 0 : it.other[f][j];
-                ha[f][j] = depth[o];
-                za[f][j] = m.bed[o];
-            }
-        if (!(dc > d.min_h)) return RC(0);
-#pragma unroll
-        for (int f = 0; f < 2; ++f) {
-            const bool two = it.other[f][1] >= 0;
-            ok[f] = it.other[f][0] >= 0 && !(ha[f][0] <= d.min_h) && !(two && ha[f][1] <= d.min_h);
-            real val = RC(0) + it.weight[f][0] * ((za[f][0] + ha[f][0]) - eta);
-            if (two) val += it.weight[f][1] * ((za[f][1] + ha[f][1]) - eta);
-            dv[f] = val / it.total[f];
-            xv[f] = it.reach[f];
-        }
+        return hang_slope(dv, xv, ok);
     }
-    if (ok[0] && ok[1]) return (dv[1] - dv[0]) / (xv[1] - xv[0]);
-    if (ok[0]) return dv[0] / xv[0];
-    if (ok[1]) return dv[1] / xv[1];
-    return RC(0);
+    real ha[2][2], za[2][2];
+#pragma unroll
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int o = it.other[f][j] < 0 ? 0 : it.other[f][j];
+            ha[f][j] = depth[o];
+            za[f][j] = m.bed[o];
+        }
+    return hang_from(it, depth[it.cell], m.bed[it.cell], ha, za, d.min_h);
 }
 
 // Both gradients of a hanging cell into d.gradients (axes it has none along
@@ -446,6 +497,28 @@ __device__ __forceinline__ real pressure_difference(const Dev &d, const real *de
         if (o1 != RC(0)) result += d.gradients[2 * m.slots[2 * index + 1] + axis] * o1;
     }
     return result;
+}
+
+// Length-weighted discharge of one face of a cell for theta < 1
+// (solver_compact.py:118-132).
+__device__ __forceinline__ real face_qn_of(const Dev &d, int ei, int face, const real *q)
+{
+    const nhf_mesh &m = d.m;
+    const int start = m.face_ptr[4 * ei + face], count = m.face_count[4 * ei + face];
+    if (count < 1) return RC(0);
+    if (count == 1) return q[m.isl_data[start]];
+    real total = RC(0), width = RC(0);
+    for (int o = 0; o < count; ++o) {
+        const int side = m.isl_data[start + o];
+        total += q[side] * m.length[side];
+        width += m.length[side];
+    }
+    return total / width;
+}
+
+__device__ __forceinline__ void face_qn_cell(const Dev &d, int ei, const real *q)
+{
+    for (int face = 0; face < 4; ++face) d.face_qn[4 * ei + face] = face_qn_of(d, ei, face, q);
 }
 
 // boundary_neighbor_sum (solver_compact.py:135-149)
@@ -526,9 +599,11 @@ struct TiledBuild {
 // does not fit the tiled form (the caller then keeps the multi-pass form).
 // tile_request: 0 picks the tile size by mesh size; 256, 512 or 1024 asks
 // for that size only. cfl_mode: 0 separate CFL pass from two waves of tiles
-// on, 1 CFL always in the step, 2 always a separate pass.
+// on, 1 CFL always in the step, 2 always a separate pass. With `resident` the
+// plan serves the resident form: its largest lists are reported there and the
+// caller checks shared memory.
 int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, size_t why_len,
-                int tile_request = 0, int cfl_mode = 0);
+                int tile_request = 0, int cfl_mode = 0, ResidentArgs *resident = nullptr);
 // Enqueue one fused step (plus the hanging/theta pre-passes and, for split
 // plans, the CFL pass). With a gate controller (256-cell tiles, split plan)
 // only the pre-passes and the gate-enabled step: the caller then enqueues
@@ -546,6 +621,23 @@ void tiled_enqueue_batch_start(const Dev &d, cudaStream_t s);
 // u, v of every cell from the caller's arrays (after a batch of the tiled or
 // lattice form has brought its state back).
 void tiled_enqueue_velocity(const Dev &d, cudaStream_t s);
+
+// The resident form: one cooperative launch per batch (nhf_resident.cu).
+struct ResidentBuild {
+    ResidentArgs args{};
+    void *tables = nullptr, *memory = nullptr;  // owned (cudaFree on destroy)
+    void *kernel = nullptr;
+    int threads = 0, patterns = 0;
+    size_t shared_bytes = 0;
+};
+// Plan it when every tile of some size can be resident at once; 0 on success,
+// else nonzero with `why` set.
+int resident_build(const nhf_mesh &m, int terms, bool theta_one, cudaStream_t s, ResidentBuild *out, char *why,
+                   size_t why_len);
+// Once the hanging gradients are laid out: the exchange flags.
+void resident_enqueue_setup(const Dev &d, const ResidentBuild &b, cudaStream_t s);
+// One batch towards words {target, origin}; the trace is in the control block.
+cudaError_t resident_enqueue_batch(const Dev &d, const ResidentBuild &b, const uint32_t words[4], cudaStream_t s);
 
 struct LatticeBuild {
     LatticePlan plan{};

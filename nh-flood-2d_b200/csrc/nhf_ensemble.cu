@@ -177,10 +177,13 @@ int nhf_ensemble_create(nhf_handle *const *members, int32_t n, int32_t grid_bloc
     if (!h0) return efail(nullptr, NHF_EINVAL, "member 0 is null");
     if (grid_blocks < -2) return efail(nullptr, NHF_EINVAL, "grid_blocks must be -2, -1, 0 or positive");
     if (grid_blocks == -2) return create_member_graphs(members, n, stream, out);
+    for (int i = 0; i < n; ++i) {
+        if (!members[i]) return efail(nullptr, NHF_EINVAL, "member %d is null", i);
+        step_plan(members[i]);
+    }
     const int tile = h0->tb.plan.tile;
     for (int i = 0; i < n; ++i) {
         const nhf_handle *h = members[i];
-        if (!h) return efail(nullptr, NHF_EINVAL, "member %d is null", i);
         if (!h->tiled) return efail(nullptr, NHF_EINVAL, "member %d is not on the fused tiled step (%s)", i, h->path.c_str());
         // the one-launch step has no gate passes: a gated member runs its own
         // batch graph in the member-graph schedule

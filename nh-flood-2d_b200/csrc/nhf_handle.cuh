@@ -30,6 +30,8 @@ struct nhf_handle {
     nhf::TiledBuild tb{};
     nhf::LatticeBuild lb{};
     bool lattice = false;
+    nhf::ResidentBuild rb{};
+    bool resident = false;      // batches of this handle run resident; its step plan (tb) is made when a graph needs it
     nhf::GateDev gate{};
     bool gate_on = false;
     void *gate_mem = nullptr;   // gate budget partials
@@ -40,6 +42,9 @@ struct nhf_handle {
 };
 
 namespace nhf {
+// The tile plan of the step-by-step form, for a handle whose own batches run
+// resident and that joins an ensemble. NHF_OK, or an error code.
+int step_plan(nhf_handle *h);
 // The ensemble's member-graph schedule (nhf_step.cu): build a member's batch
 // graph, and launch it on the member's stream after `start`, recording `done`.
 int member_graph_prepare(nhf_handle *h);

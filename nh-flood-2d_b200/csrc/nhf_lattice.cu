@@ -225,7 +225,7 @@ __device__ __noinline__ void lattice_prepare(const Dev &d, Ctl *c)
 {
     const nhf_mesh &m = d.m;
     const LatticePlan &P = d.lat;
-    clock_choose(d, c, (float)c->ndt, c->slot);
+    clock_choose(d.min_dt, c, (float)c->ndt, c->trace + c->slot * NHF_TRACE_COLS);
     if (!c->active) return;
     c->limited_cells = 0; c->limited_faces = 0;
     c->min_scale_bits = real_bits(RC(1.0));

@@ -139,27 +139,9 @@ __global__ void k_pressure(Dev d)
 
 __global__ void k_face_qn(Dev d)
 {
-    const nhf_mesh &m = d.m;
     if (!d.ctl->active) return;
     int ei = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ei >= m.e_num) return;
-    const real *q = cur_q(d, d.ctl->parity);
-    for (int dd = 0; dd < 4; ++dd) {
-        int start = m.face_ptr[4 * ei + dd], count = m.face_count[4 * ei + dd];
-        real result = RC(0.0);
-        if (count == 1) {
-            result = q[m.isl_data[start]];
-        } else if (count > 1) {
-            real total = RC(0.0), width = RC(0.0);
-            for (int o = 0; o < count; ++o) {
-                int side = m.isl_data[start + o];
-                total += q[side] * m.length[side];
-                width += m.length[side];
-            }
-            result = total / width;
-        }
-        d.face_qn[4 * ei + dd] = result;
-    }
+    if (ei < d.m.e_num) face_qn_cell(d, ei, cur_q(d, d.ctl->parity));
 }
 
 // ------------------------------------------------------------ side momentum
@@ -833,6 +815,8 @@ void enqueue_step(nhf_handle *h)
 int build_graph(nhf_handle *h)
 {
     cudaGraph_t g = nullptr;
+    int rc = step_plan(h);
+    if (rc) return rc;
     CK(h, cudaStreamBeginCapture(h->s, cudaStreamCaptureModeThreadLocal));
     k_begin<<<1, 256, 0, h->s>>>(h->dev, 0u, 0u, 0u, 0u, (h->tiled || h->lattice) ? 1 : 0);
 #ifndef NHF_REAL_DOUBLE
@@ -895,6 +879,17 @@ int build_graph(nhf_handle *h)
 }  // namespace
 
 namespace nhf {
+
+int step_plan(nhf_handle *h)
+{
+#ifndef NHF_REAL_DOUBLE
+    if (!h->resident || h->tb.device_memory) return NHF_OK;
+    char why[256] = {0};
+    h->tiled = tiled_build(h->m, h->s, &h->tb, why, sizeof(why), 0, h->p.cfl_mode) == 0;
+    if (h->tiled) h->dev.plan = h->tb.plan;   // otherwise the graph takes the multi-pass step
+#endif
+    return NHF_OK;
+}
 
 // One member's own batch graph for the ensemble's member-graph schedule: the
 // member's stream waits for `start`, runs its batch towards `target` and
@@ -982,7 +977,8 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     // Lattice form when the mesh is a uniform grid it covers (params->path 2,
     // or 0 from 2^20 cells on: on smaller grids a march of a few rows is
     // latency-bound and the tiled step is faster).
-    if (params->path == 2 || (params->path == 0 && mesh->e_num - 1 >= (1 << 20))) {
+    const bool any_form = params->path == 0 || params->path == 4;
+    if (params->path == 2 || (any_form && mesh->e_num - 1 >= (1 << 20))) {
         Dev probe{};
         probe.m = *mesh;
         probe.terms = 4 + 6 * mesh->b_num;
@@ -1001,8 +997,20 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
             h->path = std::string("multipass (lattice: ") + why + ")";
         }
     }
+    // The whole batch in one launch where one tile per SM covers the mesh (path
+    // 0, unless the caller places the CFL in a pass of its own).
+    if (!h->lattice && params->path == 0 && (params->cfl_mode == 0 || params->cfl_mode == 1)) {
+        char why[256] = {0};
+        if (resident_build(*mesh, 4 + 6 * mesh->b_num, params->sita == RC(1), h->s, &h->rb, why, sizeof(why)) == 0) {
+            h->resident = h->tiled = true;
+            char buf[160];
+            snprintf(buf, sizeof(buf), "tiled(tile=%d,patterns=%d,smem=%zu,cfl=fused,resident=%dx%d)",
+                     h->rb.args.plan.tile, h->rb.patterns, h->rb.shared_bytes, h->rb.args.plan.n_tiles, h->rb.threads);
+            h->path = buf;
+        }
+    }
     // Fused tiled step when the mesh allows it (params->path 0, or a tile size).
-    if (!h->lattice && (params->path == 0 || params->path == 3 || params->path == 256 || params->path == 512 ||
+    if (!h->lattice && !h->resident && (any_form || params->path == 3 || params->path == 256 || params->path == 512 ||
                         params->path == 1024)) {
         char why[256] = {0};
         if (params->cfl_mode < 0 || params->cfl_mode > 2) {
@@ -1010,7 +1018,7 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
             nhf_destroy(h);
             return rc;
         }
-        if (tiled_build(*mesh, h->s, &h->tb, why, sizeof(why), params->path == 3 ? 0 : params->path,
+        if (tiled_build(*mesh, h->s, &h->tb, why, sizeof(why), any_form || params->path == 3 ? 0 : params->path,
                         params->cfl_mode) == 0) {
             h->tiled = true;
             char buf[160];
@@ -1111,6 +1119,8 @@ int nhf_destroy(nhf_handle *h)
     if (h->graph_def) cudaGraphDestroy(h->graph_def);
     if (h->tb.device_memory) cudaFree(h->tb.device_memory);
     if (h->lb.device_memory) cudaFree(h->lb.device_memory);
+    if (h->rb.tables) cudaFree(h->rb.tables);
+    if (h->rb.memory) cudaFree(h->rb.memory);
     if (h->scratch) cudaFree(h->scratch);
     if (h->h_begin) cudaFreeHost(h->h_begin);
     if (h->h_trace) cudaFreeHost(h->h_trace);
@@ -1134,6 +1144,9 @@ int nhf_initialize(nhf_handle *h)
     int n = h->m.e_num > h->m.s_num ? h->m.e_num : h->m.s_num;
     k_initialize<<<grid_for(n, 256), 256, 0, h->s>>>(h->dev);
     if (h->m.hang_cells > 0) k_hang_setup<<<grid_for(2 * h->m.hang_cells, 256), 256, 0, h->s>>>(h->dev);
+#ifndef NHF_REAL_DOUBLE
+    if (h->resident) resident_enqueue_setup(h->dev, h->rb, h->s);
+#endif
     return leave(h);
 }
 
@@ -1225,9 +1238,17 @@ int nhf_run_batch_async(nhf_handle *h, const uint32_t target[2], const uint32_t 
 {
     if (!h || !target || !origin) return NHF_EINVAL;
     int rc = enter(h); if (rc) return rc;
+    uint32_t w[4] = {target[0], target[1], origin[0], origin[1]};
+#ifndef NHF_REAL_DOUBLE
+    if (h->resident) {
+        CK(h, resident_enqueue_batch(h->dev, h->rb, w, h->s));
+        CK(h, cudaMemcpyAsync(h->h_trace, h->ctl->trace, sizeof(uint32_t) * NHF_TRACE_COLS * h->p.batch_size,
+                              cudaMemcpyDeviceToHost, h->s));
+        return leave(h);
+    }
+#endif
     if (!h->graph) { rc = build_graph(h); if (rc) return rc; }
     Dev d = h->dev;
-    uint32_t w[4] = {target[0], target[1], origin[0], origin[1]};
     int prepare_first = (h->tiled || h->lattice) ? 1 : 0;
     void *args[6] = {&d, &w[0], &w[1], &w[2], &w[3], &prepare_first};
     cudaKernelNodeParams kp = h->begin_params;

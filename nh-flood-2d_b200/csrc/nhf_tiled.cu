@@ -947,6 +947,7 @@ struct HostMesh {
     int e, s;
     std::vector<int32_t> topo, fptr, fcnt, isl;
     std::vector<uint8_t> sbf;
+    std::vector<int32_t> edge;  // hanging edge of each side (resident plans of meshes with hanging edges)
 };
 
 int copy_back(const nhf_mesh &m, cudaStream_t st, HostMesh &hm)
@@ -996,7 +997,7 @@ bool consistent(const HostMesh &hm, std::string &why)
 
 int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::vector<int32_t> &tile_pattern,
                std::vector<int32_t> &tile_cbase, std::vector<int32_t> &tile_sbase, int &max_ext, int &max_sides,
-               int &max_faces, int rings, std::string &why)
+               int &max_faces, int rings, std::string &why, ResidentArgs *resident)
 {
     const int e = hm.e, s = hm.s;
     // cell adjacency through interior sides
@@ -1114,6 +1115,18 @@ int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::v
         if (p.fidx.size() > 65535) { why = "tile face table too large"; return 1; }
         p.counts[8] = (int)p.fidx.size();
         max_faces = std::max(max_faces, (int)p.fidx.size());
+        if (resident) {
+            int hang = 0;
+            if (!hm.edge.empty())
+                for (int sid : sides) hang += hm.edge[sid] >= 0 ? 1 : 0;
+            resident->max_hang = std::max(resident->max_hang, hang);
+            resident->max_don = std::max(resident->max_don, n_don);
+            resident->max_owned = std::max(resident->max_owned, n_owned);
+            resident->max_r1 = std::max(resident->max_r1, n_r01 - n_r0);
+            for (int i = 1; i <= n_r0; ++i)
+                for (int dd = 0; dd < 4; ++dd)
+                    resident->max_per_face = std::max(resident->max_per_face, hm.fcnt[4 * ext[i] + dd]);
+        }
         max_ext = std::max(max_ext, (int)ext.size());
         max_sides = std::max(max_sides, (int)sides.size());
         uint64_t hsh = pattern_hash(p);
@@ -1186,34 +1199,11 @@ __global__ void k_pressure_tiled(const __grid_constant__ Dev d)
     if (slot < d.m.hang_cells) hang_slot(d, slot);
 }
 
-// length-weighted face discharge for theta < 1 (solver_compact.py:118-132)
-__device__ __forceinline__ void face_qn_cell(const Dev &d, int ei)
-{
-    const nhf_mesh &m = d.m;
-    const float *q = cur_q(d, d.ctl->parity);
-    for (int dd = 0; dd < 4; ++dd) {
-        int start = m.face_ptr[4 * ei + dd], count = m.face_count[4 * ei + dd];
-        float result = 0.0f;
-        if (count == 1) {
-            result = q[m.isl_data[start]];
-        } else if (count > 1) {
-            float total = 0.0f, width = 0.0f;
-            for (int o = 0; o < count; ++o) {
-                int side = m.isl_data[start + o];
-                total += q[side] * m.length[side];
-                width += m.length[side];
-            }
-            result = total / width;
-        }
-        d.face_qn[4 * ei + dd] = result;
-    }
-}
-
 __global__ void k_face_qn_tiled(const __grid_constant__ Dev d)
 {
     if (!d.ctl->active) return;
     int ei = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ei < d.m.e_num) face_qn_cell(d, ei);
+    if (ei < d.m.e_num) face_qn_cell(d, ei, cur_q(d, d.ctl->parity));
 }
 
 // ------------------------------------------------------- ensemble kernels
@@ -1259,7 +1249,8 @@ __global__ void k_ens_face_qn(const Dev *devs, const int2 *items)
     const Dev &d = devs[w.x];
     if (!d.ctl->active) return;
     const int end = min(d.m.e_num, (w.y + 1) * kEnsChunk);
-    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x) face_qn_cell(d, i);
+    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x)
+        face_qn_cell(d, i, cur_q(d, d.ctl->parity));
 }
 
 // CFL pass of every member: items are (member, chunk of kEnsChunk sides);
@@ -1313,7 +1304,7 @@ __global__ void k_ens_finish(const Dev *devs, uint32_t *trace, int batch)
 }  // namespace
 
 int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, size_t why_len, int tile_request,
-                int cfl_mode)
+                int cfl_mode, ResidentArgs *resident)
 {
     std::string reason;
     auto bad = [&](const std::string &r) {
@@ -1324,6 +1315,12 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     HostMesh hm;
     if (copy_back(m, s, hm)) return bad("copying the mesh tables to the host failed");
     if (!consistent(hm, reason)) return bad(reason);
+    if (resident && m.hang_cells > 0) {
+        hm.edge.resize((size_t)m.s_num);
+        if (cudaMemcpyAsync(hm.edge.data(), m.edge_index, 4 * hm.edge.size(), cudaMemcpyDeviceToHost, s) ||
+            cudaStreamSynchronize(s))
+            return bad("copying the mesh tables to the host failed");
+    }
     std::vector<Pattern> patterns;
     std::vector<int32_t> tp, tc, ts;
     int max_ext = 0, max_sides = 0, max_faces = 0, tile = 0;
@@ -1336,7 +1333,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     if (m.e_num < 148 * 2 * 1024 || m.hang_cells > 0) sizes = {256, 512, 1024};
     else if (m.e_num < 148 * 4 * 1024) sizes = {512, 256};
     if (tile_request) {
-        if (tile_request != 256 && tile_request != 512 && tile_request != 1024)
+        if (!resident && tile_request != 256 && tile_request != 512 && tile_request != 1024)
             return bad("tile size must be 256, 512 or 1024");
         sizes = {tile_request};
     }
@@ -1345,10 +1342,11 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         // The separate CFL pass pays one launch per step for less halo work
         // (no ring 3, no ring-1 depth recompute): worth it from two waves of
         // resident blocks on.
-        const int resident = 148 * (T == 256 ? kMinBlocks<256> : kMinBlocks<512>);
+        const int wave = 148 * (T == 256 ? kMinBlocks<256> : kMinBlocks<512>);
         const int n_tiles = (m.e_num + T - 1) / T;
-        split = cfl_mode == 2 || (cfl_mode == 0 && n_tiles >= 2 * resident);
-        if (plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason))
+        split = cfl_mode == 2 || (cfl_mode == 0 && n_tiles >= 2 * wave);
+        if (plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason,
+                       resident))
             return bad(reason);
         // The budget reduction stages one term of every thread (NT doubles)
         // in the 24 * max_ext bytes of shared arrays that are dead after the
@@ -1356,7 +1354,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         const int nt = T == 256 ? 256 : 512;
         if (24 * max_ext < 8 * nt) max_ext = (8 * nt + 23) / 24;
         smem = (size_t)max_ext * 32 + (size_t)max_sides * 16 + (size_t)max_faces * 2 + 16;
-        if (smem <= (size_t)kMaxSharedBytes) { tile = T; break; }
+        if (resident || smem <= (size_t)kMaxSharedBytes) { tile = T; break; }
     }
     if (!tile) return bad("tile halos exceed shared memory (cell numbering is not spatially coherent)");
     // flatten patterns
@@ -1422,6 +1420,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     out->device_memory = mem;
     out->shared_bytes = smem;
     out->patterns = (int)patterns.size();
+    if (resident) return 0;
     if (tile == 1024) set_smem_all<512, 2>(smem);
     else if (tile == 512) set_smem_all<512, 1>(smem);
     else set_smem_all<256, 1>(smem);

@@ -42,8 +42,12 @@ MEMBER_GRAPHS = -2  # nhf_ensemble_create's grid_blocks for the member-graph sch
 
 
 def plain_factory(device: str = 'cuda:0'):
-    """Engines with the plain form's own step choice."""
+    """Engines with the plain form's own step choice, but for the resident
+    form: one member's resident batch holds every SM it runs on, so members
+    would run one after another."""
     def factory(arrays, params):
+        if params.path == 'auto' and arrays.gate is None:
+            params.path = 'steps'
         return CudaEngine(arrays, params, device=device)
     return factory
 

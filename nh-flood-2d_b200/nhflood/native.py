@@ -141,9 +141,9 @@ def exported_symbols() -> list[str]:
 
 
 def path_code(path) -> int:
-    """nhf_params.path for a StepParams.path: 'auto', 'multipass', 'lattice'
-    (uniform grids), 'tiled' (the fused tiled step, tile size by mesh size)
-    or 'tile256' / 'tile512' / 'tile1024' (fused step with that tile size)."""
+    """nhf_params.path for a StepParams.path: 'auto', 'steps' (as 'auto', but
+    never the resident form), 'multipass', 'lattice' (uniform grids), 'tiled'
+    (the fused tiled step, tile size by mesh size) or 'tile256' / 'tile512' / 'tile1024' (fused step with that tile size)."""
     if path == 'auto':
         return 0
     if path == 'multipass':
@@ -152,6 +152,8 @@ def path_code(path) -> int:
         return 2
     if path == 'tiled':
         return 3
+    if path == 'steps':
+        return 4
     if isinstance(path, str) and path.startswith('tile') and path[4:] in ('256', '512', '1024'):
         return int(path[4:])
     raise ValueError(f'unknown step path {path!r}')
