@@ -110,10 +110,10 @@ typedef struct nhf_params {
     nhf_real min_h;   /* wet threshold */
     float min_dt;     /* F32(1e-4) CFL floor (solver_compact.py:31) */
     int32_t batch_size; /* steps per batch, 1..64 (clock.py:48-51) */
-    int32_t path;       /* 0: the lattice form on a uniform grid it covers
-                           of at least 2^20 cells, else the resident form
-                           (the whole batch in one cooperative launch) when
-                           one tile per SM covers the mesh, else the fused
+    int32_t path;       /* 0: the resident form (the whole batch in one
+                           cooperative launch) when one tile per SM covers
+                           the mesh, else the lattice form on a uniform grid
+                           it covers of at least 2^18 cells, else the fused
                            tiled step when the mesh allows it, else
                            multi-pass; 4: the same without the resident form
                            (members of an ensemble, which run beside others); 1: always the multi-pass step;

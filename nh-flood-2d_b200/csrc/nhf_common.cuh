@@ -48,6 +48,7 @@ struct Ctl {
     uint32_t trace[NHF_MAX_BATCH * NHF_TRACE_COLS];
     unsigned long long cfl_min_bits;  // FP64 build: the CFL minimum's bits, then
     int32_t cfl_arg_min;              // the lowest side id that attains it
+    unsigned long long dry_key;       // the least CFL key of an all-dry state (initialize)
     uint32_t epoch, batches;          // resident form: steps and batches so far
     int32_t stalled;                  // resident form: a wait ran out
 };
@@ -90,8 +91,8 @@ struct ResidentArgs {
 // "v" side, the south face its "h" side.
 struct LatticePlan {
     int32_t nx, ny, lx, ly, strips, chunks, rows, block_warps, min_blocks, rain_cells, horton;
-    int32_t buffer_stride;          // elements from the first to the second buffer of h, qv and qh
     real sdc_v, sdc_h, len_v, len_h, area, width, height;
+    real inv_sdc_v, inv_sdc_h, inv_area;  // exact inverses of powers of two, else 0
     const int32_t *cell;            // [lx*ly] global cell id (0: hole, border, padding)
     const int32_t *side_v, *side_h; // [lx*ly] global id of the west / south side (0: none)
     const uint8_t *live;            // [lx*ly] 1 for a real cell
@@ -100,12 +101,15 @@ struct LatticePlan {
     real *h[2], *qv[2], *qh[2];     // double-buffered depth and side discharges
     real *z, *nv, *nh;              // bed (refreshed each batch), Manning n of the sides
     int16_t *bi;                    // boundary id, -1 for none
-    int32_t *rain;                  // rain pixel (rain_cells only)
+    real *rate;                     // rain rate, refreshed each batch (rain_cells only)
     real *rain_time, *infil, *max_depth, *max_speed;
     uint32_t *peak_hi, *peak_lo;
     real *f0, *fc, *k;              // Horton (horton only)
     float *terms;                   // [terms][e_num] budget terms of a step by global id, else zero
-    uint32_t *touched;              // [blocks] terms some cell of a 256-cell budget block holds
+    uint32_t *touched;              // [blocks] terms but 0 some cell of a 256-cell budget block holds
+    uint8_t *touched_rain;          // [blocks] 1 where some cell holds term 0 (infiltration)
+    int32_t *odd;                   // 1 during a batch that starts with extrema below zero
+    uint8_t *plain;                 // [chunks*strips] 1: the warp's cells are live and off the boundaries
     uint32_t *part;                 // [4][strips*chunks] per-warp limited cells, limited faces, wet cells, min scale bits
     unsigned long long *part_cfl;   // [strips*chunks] per-warp CFL key
     float4 *edge_first;             // [strips][chunks*rows] first column: new depth, bed, west discharge, live
@@ -157,6 +161,11 @@ __device__ __forceinline__ float maxf(float a, float b) { return a > b ? a : b; 
 __device__ __forceinline__ float minf(float a, float b) { return b < a ? b : a; }
 __device__ __forceinline__ real rmax(real a, real b) { return a > b ? a : b; }
 __device__ __forceinline__ real rmin(real a, real b) { return b < a ? b : a; }
+// rmax with a constant that is neither NaN nor -0: one instruction instead of a
+// compare and a select, and the same bits (a NaN gives the constant, -0 and +0
+// give +0).
+__device__ __forceinline__ float rmaxc(float a, float c) { return fmaxf(a, c); }
+__device__ __forceinline__ double rmaxc(double a, double c) { return fmax(a, c); }
 
 __device__ __forceinline__ const real *cur_depth(const Dev &d, int parity) { return parity ? d.depth_b : d.m.depth; }
 __device__ __forceinline__ const real *cur_q(const Dev &d, int parity) { return parity ? d.q_b : d.m.q; }
@@ -651,7 +660,8 @@ int lattice_build(const Dev &d, cudaStream_t s, LatticeBuild *out, char *why, si
 void lattice_enqueue_batch_start(const Dev &d, cudaStream_t s);
 // One step: the fused lattice step, then the pass that reduces its budget
 // blocks, takes the CFL candidate, commits the step and prepares the next.
-void lattice_enqueue_step(const Dev &d, cudaStream_t s);
+// `step` is the step's number in the batch.
+void lattice_enqueue_step(const Dev &d, int step, cudaStream_t s);
 void lattice_enqueue_batch_end(const Dev &d, cudaStream_t s);
 
 // Ensemble form: several meshes (members) on the fused tiled step with one

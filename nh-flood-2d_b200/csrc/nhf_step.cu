@@ -94,6 +94,24 @@ __global__ void k_prepare(Dev d)
 
 // ------------------------------------------------------ pressure (pressure.py)
 
+#ifndef NHF_REAL_DOUBLE
+// The least CFL key (dt bits << 32 | side id) of an all-dry state: every
+// interior side at the face depth's floor without discharge.
+__global__ void k_dry_key(Dev d)
+{
+    const nhf_mesh &m = d.m;
+    unsigned long long best = kCflEmpty;
+    for (int si = blockIdx.x * blockDim.x + threadIdx.x + 1; si < m.s_num; si += gridDim.x * blockDim.x) {
+        if (m.topology[3 * si + 1] == 0 || m.topology[3 * si + 2] == 0) continue;
+        const unsigned long long key =
+            ((unsigned long long)__float_as_uint(cfl_value(d.afa, d.g, m.length[si], RC(0), RC(0.01))) << 32) | (unsigned)si;
+        best = key < best ? key : best;
+    }
+    best = warp_min_key(best);
+    if ((threadIdx.x & 31) == 0 && best != kCflEmpty) atomicMin(&d.ctl->dry_key, best);
+}
+#endif
+
 // The hanging-edge gradients' inputs from the mesh tables, once per solve; a
 // thread per (cell, axis). Sums run in the order hang_face takes them.
 __global__ void k_hang_setup(Dev d)
@@ -822,7 +840,7 @@ int build_graph(nhf_handle *h)
 #ifndef NHF_REAL_DOUBLE
     if (h->lattice) {
         lattice_enqueue_batch_start(h->dev, h->s);
-        for (int i = 0; i < h->p.batch_size; ++i) lattice_enqueue_step(h->dev, h->s);
+        for (int i = 0; i < h->p.batch_size; ++i) lattice_enqueue_step(h->dev, i, h->s);
         lattice_enqueue_batch_end(h->dev, h->s);
     } else if (h->tiled) {
         tiled_enqueue_batch_start(h->dev, h->s);
@@ -974,11 +992,24 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
 #ifdef NHF_REAL_DOUBLE
     h->path = "multipass (FP64 build)";
 #else
-    // Lattice form when the mesh is a uniform grid it covers (params->path 2,
-    // or 0 from 2^20 cells on: on smaller grids a march of a few rows is
-    // latency-bound and the tiled step is faster).
     const bool any_form = params->path == 0 || params->path == 4;
-    if (params->path == 2 || (any_form && mesh->e_num - 1 >= (1 << 20))) {
+    // The whole batch in one launch where one tile per SM covers the mesh (path
+    // 0, unless the caller places the CFL in a pass of its own).
+    if (params->path == 0 && (params->cfl_mode == 0 || params->cfl_mode == 1)) {
+        char why[256] = {0};
+        if (resident_build(*mesh, 4 + 6 * mesh->b_num, params->sita == RC(1), h->s, &h->rb, why, sizeof(why)) == 0) {
+            h->resident = h->tiled = true;
+            char buf[160];
+            snprintf(buf, sizeof(buf), "tiled(tile=%d,patterns=%d,smem=%zu,cfl=fused,resident=%dx%d)",
+                     h->rb.args.plan.tile, h->rb.patterns, h->rb.shared_bytes, h->rb.args.plan.n_tiles, h->rb.threads);
+            h->path = buf;
+        }
+    }
+    // Lattice form when the mesh is a uniform grid it covers (params->path 2, or
+    // a grid of at least 2^18 cells that does not run resident: 600 x 600 cells
+    // 1357 us per 32 steps against 1603 on tiles, 1003 x 741 2047 against 2806
+    // (numbered by rows 2054 against 4580), 421 x 307 1037 against 983).
+    if (!h->resident && (params->path == 2 || (any_form && mesh->e_num - 1 >= (1 << 18)))) {
         Dev probe{};
         probe.m = *mesh;
         probe.terms = 4 + 6 * mesh->b_num;
@@ -995,18 +1026,6 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
         } else {
             if (h->lb.device_memory) { cudaFree(h->lb.device_memory); h->lb.device_memory = nullptr; }
             h->path = std::string("multipass (lattice: ") + why + ")";
-        }
-    }
-    // The whole batch in one launch where one tile per SM covers the mesh (path
-    // 0, unless the caller places the CFL in a pass of its own).
-    if (!h->lattice && params->path == 0 && (params->cfl_mode == 0 || params->cfl_mode == 1)) {
-        char why[256] = {0};
-        if (resident_build(*mesh, 4 + 6 * mesh->b_num, params->sita == RC(1), h->s, &h->rb, why, sizeof(why)) == 0) {
-            h->resident = h->tiled = true;
-            char buf[160];
-            snprintf(buf, sizeof(buf), "tiled(tile=%d,patterns=%d,smem=%zu,cfl=fused,resident=%dx%d)",
-                     h->rb.args.plan.tile, h->rb.patterns, h->rb.shared_bytes, h->rb.args.plan.n_tiles, h->rb.threads);
-            h->path = buf;
         }
     }
     // Fused tiled step when the mesh allows it (params->path 0, or a tile size).
@@ -1103,6 +1122,7 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     init.cfl_packed = kCflEmpty;
     init.ndt = RC(0);
     init.cfl_min_bits = kCflEmpty;
+    init.dry_key = kCflEmpty;
     init.cfl_arg_min = mesh->s_num;
     CKC(cudaMemcpyAsync(h->ctl, &init, sizeof(Ctl), cudaMemcpyHostToDevice, h->s));
     CKC(cudaStreamSynchronize(h->s));
@@ -1145,6 +1165,7 @@ int nhf_initialize(nhf_handle *h)
     k_initialize<<<grid_for(n, 256), 256, 0, h->s>>>(h->dev);
     if (h->m.hang_cells > 0) k_hang_setup<<<grid_for(2 * h->m.hang_cells, 256), 256, 0, h->s>>>(h->dev);
 #ifndef NHF_REAL_DOUBLE
+    k_dry_key<<<148 * 4, 256, 0, h->s>>>(h->dev);
     if (h->resident) resident_enqueue_setup(h->dev, h->rb, h->s);
 #endif
     return leave(h);
