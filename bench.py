@@ -98,6 +98,10 @@ def launches_per_batch(run) -> int:
     pre = (1 if run.arrays.hang_cells else 0) + (0 if run.w.sita == 1.0 else 1)
     gate = run.arrays.gate
     once = 0
+    if 'edges=' in eng.path and gate is None and run.arrays.hang_cells:
+        # the pass after a step takes the next step's gradients; the first step's have a launch
+        pre -= 1
+        once += 1
     if gate is not None:
         if tiled:  # exchange volumes with the end motion; start motion in the CFL pass (own launch at batch start)
             pre += 1

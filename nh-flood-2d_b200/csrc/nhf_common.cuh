@@ -48,6 +48,7 @@ struct Ctl {
     uint32_t trace[NHF_MAX_BATCH * NHF_TRACE_COLS];
     unsigned long long cfl_min_bits;  // FP64 build: the CFL minimum's bits, then
     int32_t cfl_arg_min;              // the lowest side id that attains it
+    int32_t grad_parity;              // tiled form: 1 when the last step's gradients are in the second buffer
     unsigned long long dry_key;       // the least CFL key of an all-dry state (initialize)
     uint32_t epoch, batches;          // resident form: steps and batches so far
     int32_t stalled;                  // resident form: a wait ran out
@@ -59,12 +60,15 @@ struct TilePlan {
     int32_t split;  // 1: two halo rings and a separate CFL pass; 0: three rings, CFL in the step
     // per tile: n_ext, n_r0, n_r01, n_don, n_sides, n_owned, n_qf, r0_first_offset,
     // n_faces, cbase, sbase, then the pattern's ext, side, face_desc and face_idx offsets, 0
+    int32_t stage_sdn;         // 1: centre distance and Manning n are staged in shared memory
+    int32_t n_edges;           // split plans: interior sides between tiles
+    const int4 *edges;         // [n_edges] lower cell, higher cell, side, 0
     const int4 *tile_head;     // [n_tiles][4]
     const int32_t *ext_rel;    // relative cell ids by local slot (slot 0 = exterior sentinel)
     const int32_t *side_rel;   // relative side ids by local side
-    const uint32_t *side_lohi; // local slots: lower | higher << 16
+    const uint32_t *side_lohi; // local slots: lower | 0x8000 on hanging sides (not in resident plans) | higher << 16
     const uint32_t *face_desc; // per slot 0..n_r012: start | counts (4 x 4 bits) << 16
-    const uint16_t *face_idx;  // local side indices in the reference's CSR order
+    const uint16_t *face_idx;  // local side indices in the reference's CSR order, each cell's from an 8-byte boundary
 };
 
 // What the resident form (nhf_resident.cu) adds to a tile plan of three rings:
@@ -150,7 +154,8 @@ struct Dev {
     real *values, *level_values, *rain_rates, *sdc, *donor_scale, *face_qn, *eq, *gradients;
     double *acc_sum, *acc_comp;
     // second buffers of the double-buffered state (tiled form)
-    real *depth_b, *q_b, *rain_time_b;
+    real *depth_b, *q_b, *rain_time_b, *gradients_b;
+    real *rain_rate;  // [e_num] rain rate of each cell during a batch (tiled form)
     HangItem *hang;  // [hang_cells][2] (filled by initialize)
     float2 *sdn;  // per side {centre distance, Manning n} (tiled form; filled by initialize)
     TilePlan plan;
@@ -613,11 +618,12 @@ struct TiledBuild {
 // caller checks shared memory.
 int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, size_t why_len,
                 int tile_request = 0, int cfl_mode = 0, ResidentArgs *resident = nullptr);
-// Enqueue one fused step (plus the hanging/theta pre-passes and, for split
-// plans, the CFL pass). With a gate controller (256-cell tiles, split plan)
+// Enqueue one fused step, number `step` of its batch (plus the hanging/theta
+// pre-passes and, for split plans, the pass that takes the CFL between tiles and
+// the next step's gradients). With a gate controller (256-cell tiles, split plan)
 // only the pre-passes and the gate-enabled step: the caller then enqueues
 // the controller's passes and tiled_enqueue_cfl.
-void tiled_enqueue_step(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate = nullptr);
+void tiled_enqueue_step(const Dev &d, const TiledBuild &b, int step, cudaStream_t s, const GateDev *gate = nullptr);
 // The separate CFL pass of a split plan (nothing otherwise); with a gate
 // controller its last block also runs the next step's check_gates.
 void tiled_enqueue_cfl(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate = nullptr);

@@ -889,6 +889,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
         c->active = ck.active; c->slot = batch;
         c->ndt = sh_ndt; c->cfl_arg = sh_arg;
         c->epoch = epoch;
+        if (epoch != epoch0) c->grad_parity = 0;
         c->batches += 1;
         c->done_blocks = 0;
     }

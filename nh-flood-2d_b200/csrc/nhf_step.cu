@@ -150,6 +150,7 @@ __global__ void k_pressure(Dev d)
 {
     if (!d.ctl->active) return;
     int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot == 0) d.ctl->grad_parity = 0;
     if (slot < d.m.hang_cells) hang_slot(d, slot);
 }
 
@@ -726,6 +727,13 @@ __global__ void k_cfl_edge(Dev d, real *out)
     *reinterpret_cast<int32_t *>(out + 2) = c->cfl_arg;
 }
 
+// The last step's hanging-edge gradients.
+__global__ void k_gradients(Dev d, real *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 2 * d.m.hang_cells) out[i] = (d.ctl->grad_parity ? d.gradients_b : d.gradients)[i];
+}
+
 // eq_t from the current discharges (solver_compact.py:548-559 face sums)
 __global__ void k_eq(Dev d)
 {
@@ -850,7 +858,7 @@ int build_graph(nhf_handle *h)
                 // runs it for the next ones), the step with the source terms,
                 // the exchange volumes with finish_gate_bed, the CFL pass
                 if (i == 0) k_gate_move<<<1, 256, 0, h->s>>>(h->dev, h->gate, 0);
-                tiled_enqueue_step(h->dev, h->tb, h->s, &h->gate);
+                tiled_enqueue_step(h->dev, h->tb, i, h->s, &h->gate);
                 // the exchange volumes and finish_gate_bed in one launch
                 if (h->gate.n_flux > 0)
                     k_gate_flux<<<grid_for(h->gate.n_flux, kBlock), kBlock, 0, h->s>>>(h->dev, h->gate, 1);
@@ -858,7 +866,7 @@ int build_graph(nhf_handle *h)
                     k_gate_move<<<1, 256, 0, h->s>>>(h->dev, h->gate, 1);
                 tiled_enqueue_cfl(h->dev, h->tb, h->s, &h->gate);
             } else {
-                tiled_enqueue_step(h->dev, h->tb, h->s);
+                tiled_enqueue_step(h->dev, h->tb, i, h->s);
             }
         }
         tiled_enqueue_batch_end(h->dev, h->s);
@@ -1041,8 +1049,10 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
                         params->cfl_mode) == 0) {
             h->tiled = true;
             char buf[160];
-            snprintf(buf, sizeof(buf), "tiled(tile=%d,patterns=%d,smem=%zu,cfl=%s)", h->tb.plan.tile,
-                     h->tb.patterns, h->tb.shared_bytes, h->tb.plan.split ? "pass" : "fused");
+            snprintf(buf, sizeof(buf), "tiled(tile=%d,patterns=%d,smem=%zu,cfl=%s", h->tb.plan.tile, h->tb.patterns,
+                     h->tb.shared_bytes, h->tb.plan.split ? "pass" : "fused");
+            if (h->tb.plan.split) snprintf(buf + strlen(buf), sizeof(buf) - strlen(buf), ",edges=%d", h->tb.plan.n_edges);
+            strcat(buf, ")");
             h->path = buf;
         } else {
             h->path = std::string("multipass (") + why + ")";
@@ -1069,6 +1079,8 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     size_t o_db = h->tiled ? take(sizeof(real) * (size_t)e) : 0;
     size_t o_qb = h->tiled ? take(sizeof(real) * (size_t)sn) : 0;
     size_t o_rb = h->tiled ? take(sizeof(real) * (size_t)e) : 0;
+    size_t o_rr = h->tiled ? take(sizeof(real) * (size_t)e) : 0;
+    size_t o_gb = h->tiled ? take(sizeof(real) * 2 * hc) : 0;
     size_t o_sdn = h->tiled ? take(sizeof(float2) * (size_t)sn) : 0;
     CKC(cudaMalloc(&h->scratch, off));
     CKC(cudaMemsetAsync(h->scratch, 0, off, h->s));
@@ -1110,6 +1122,8 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
         d.depth_b = (real *)(base + o_db);
         d.q_b = (real *)(base + o_qb);
         d.rain_time_b = (real *)(base + o_rb);
+        d.rain_rate = (real *)(base + o_rr);
+        d.gradients_b = (real *)(base + o_gb);
         d.sdn = (float2 *)(base + o_sdn);
         d.plan = h->tb.plan;
     }
@@ -1482,8 +1496,7 @@ int nhf_read_gradients(nhf_handle *h, nhf_real *gradients)
     if (!h || !gradients) return NHF_EINVAL;
     if (h->m.hang_cells <= 0) return NHF_OK;
     int rc = enter(h); if (rc) return rc;
-    CK(h, cudaMemcpyAsync(gradients, h->dev.gradients, sizeof(real) * 2 * (size_t)h->m.hang_cells,
-                          cudaMemcpyDeviceToDevice, h->s));
+    k_gradients<<<grid_for(2 * h->m.hang_cells, 256), 256, 0, h->s>>>(h->dev, gradients);
     return leave(h);
 }
 

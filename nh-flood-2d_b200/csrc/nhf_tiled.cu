@@ -9,10 +9,13 @@
 //   ring <= 3  water level and bed           -> momentum q* of faces(ring <= 2)
 //   ring <= 2  donor factor from those q*    -> final q of faces(ring <= 1)
 //   ring <= 1  depth update from final q     -> CFL of the sides the tile owns
-// That is the fused-CFL form. On meshes of several waves of tiles the plan
-// drops ring 3 and the ring-1 depth recompute, and the CFL candidate of the
-// next step is a separate grid-wide pass on the new state (k_cfl_tiled): the
-// halo work saved outweighs one more launch per step (TilePlan::split).
+// That is the fused-CFL form. On meshes of several waves of tiles and on those
+// with hanging edges the plan drops ring 3 and the ring-1 depth recompute: the
+// step takes the CFL of the sides inside its tile and a pass after it
+// (k_edges_tiled) that of the sides between tiles, with the next step's
+// hanging-edge gradients. The halo work saved outweighs the launch
+// (TilePlan::split). Gate runs, which move beds in between, and ensemble
+// launches keep a pass over all sides.
 // Every quantity is computed with the reference's operation order, so a cell
 // that several tiles recompute gets the same bits everywhere; each output
 // (depth, side q, extrema, budget block) has exactly one writer, its owner
@@ -41,7 +44,7 @@
 namespace nhf {
 namespace {
 
-constexpr int kMaxSharedBytes = 108 * 1024;
+constexpr int kMaxSharedBytes = 108 * 1024;   // two blocks per SM
 // Resident blocks per SM the register budget is sized for: 5 x 256 threads
 // (48 registers) for 256-cell tiles, 2 x 512 threads (64) for larger ones.
 template <int NT>
@@ -60,6 +63,18 @@ __device__ __forceinline__ void cp_async4(void *smem, const void *gmem)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -76,30 +91,66 @@ struct CellTerms {
 struct Tile {
     int n_ext, n_r0, n_r01, n_don, n_sides, n_owned, n_qf, r0off, n_faces;
     int cbase, sbase;
-    const int32_t *ext;
-    const int32_t *srel;
-    const uint32_t *lohi;
-    const uint32_t *fdesc;
-    const uint16_t *fidx;
 };
 
+// A local side is its lower slot (15 bits), a flag for the sides whose level
+// difference takes hanging gradients, and its higher slot.
+constexpr uint32_t kSlot = 0x7fffu, kHangSide = 0x8000u;
+// Faces of one side each, west, east, south, north (face_desc's counts).
+constexpr uint32_t kSingle = 0x1111u;
+
 // Face flux sums of one local cell (solver_compact.py:548-557) in the
-// reference's CSR order.
-__device__ __forceinline__ void face_sums(const Tile &tl, const float *sh_q, const float *sh_len, int slot,
+// reference's CSR order. Most cells have one side per face: their four side
+// indices are one 8-byte load (the planner aligns each cell's list).
+__device__ __forceinline__ void face_sums(uint32_t fd, const uint16_t *fidx, const float *sh_q, const float *sh_len,
                                           float fl[4])
 {
-    uint32_t fd = tl.fdesc[slot];
+    const uint32_t counts = fd >> 16;
     int k = (int)(fd & 0xffffu);
-    uint32_t counts = fd >> 16;
+    if (counts == kSingle) {
+        const uint2 w = *reinterpret_cast<const uint2 *>(fidx + k);
+        const uint32_t ls[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
+#pragma unroll
+        for (int dd = 0; dd < 4; ++dd) fl[dd] = 0.0f + sh_q[ls[dd]] * sh_len[ls[dd]];
+        return;
+    }
     for (int dd = 0; dd < 4; ++dd) {
         int cnt = (int)((counts >> (4 * dd)) & 15u);
         float face_flux = 0.0f;
         for (int j = 0; j < cnt; ++j) {
-            int ls = tl.fidx[k++];
+            int ls = fidx[k++];
             face_flux += sh_q[ls] * sh_len[ls];
         }
         fl[dd] = face_flux;
     }
+}
+
+// Outflow of one local cell over a step (solver_compact.py:500-508) added to
+// `outgoing`, side by side in the same order.
+__device__ __forceinline__ float face_outflow(uint32_t fd, const uint16_t *fidx, const float *sh_q,
+                                              const float *sh_len, float dt, float outgoing)
+{
+    const uint32_t counts = fd >> 16;
+    int k = (int)(fd & 0xffffu);
+    if (counts == kSingle) {
+        const uint2 w = *reinterpret_cast<const uint2 *>(fidx + k);
+        const uint32_t ls[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
+#pragma unroll
+        for (int dd = 0; dd < 4; ++dd) {
+            const float out = sh_q[ls[dd]] * sh_len[ls[dd]];
+            outgoing += rmaxc((dd & 1) ? out : -out, 0.0f) * dt;
+        }
+        return outgoing;
+    }
+    for (int dd = 0; dd < 4; ++dd) {
+        const int cnt = (int)((counts >> (4 * dd)) & 15u);
+        for (int j = 0; j < cnt; ++j) {
+            const int ls = fidx[k++];
+            const float out = sh_q[ls] * sh_len[ls];
+            outgoing += rmaxc((dd & 1) ? out : -out, 0.0f) * dt;
+        }
+    }
+    return outgoing;
 }
 
 // The canonical 256-slot pairwise tree (stride 128 .. 1) run on every
@@ -142,13 +193,31 @@ __device__ __forceinline__ float term_value(int t, int B, float removed, float f
 
 // CFL candidate (solver_compact.py:628-631) of an interior side with face depth
 // h, folded into the running minimum key (dt bits << 32 | side id); the exact
-// value is formed only where it may be at or below the minimum.
+// value is formed only where it may be at or below the minimum. A side at the
+// face depth's floor with no discharge is left to the dry key (the least key
+// of an all-dry state, folded in with the result): no side's value is above
+// its dry one, so where the minimum is that small the dry key's sides attain it.
 __device__ __forceinline__ void fold_cfl(const Dev &d, float len, float q, float h, unsigned gid,
                                          unsigned long long &best)
 {
+    if (h == 0.01f && q == 0.0f) return;
     if (cfl_above(d.afa * len, d.g, q, h, __uint_as_float((uint32_t)(best >> 32)))) return;
     const unsigned long long key = ((unsigned long long)__float_as_uint(cfl_value(d.afa, d.g, len, q, h)) << 32) | gid;
     best = key < best ? key : best;
+}
+
+// The step's CFL result: the least of the blocks' keys and the dry key.
+__device__ __forceinline__ void set_cfl(Ctl *c)
+{
+    const unsigned long long all = atomicExch(&c->cfl_packed, kCflEmpty);
+    const unsigned long long packed = c->dry_key < all ? c->dry_key : all;
+    if (packed == kCflEmpty) {
+        c->ndt = __uint_as_float(0x7f800000u);
+        c->cfl_arg = 0;
+    } else {
+        c->ndt = __uint_as_float((uint32_t)(packed >> 32));
+        c->cfl_arg = (int32_t)(packed & 0xffffffffu);
+    }
 }
 
 // One fused step of tile t of the mesh described by d (n_tiles tiles).
@@ -191,17 +260,22 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     }
     const int parity = c->parity;
     const float dt = c->dt;
-    const int raining = c->raining;
     const float *depth_in = parity ? d.depth_b : m.depth;
     float *depth_out = parity ? m.depth : d.depth_b;
     const float *q_in = parity ? d.q_b : m.q;
     float *q_out = parity ? m.q : d.q_b;
     const float *rt_in = parity ? d.rain_time_b : m.rain_time;
     float *rt_out = parity ? m.rain_time : d.rain_time_b;
+    // the split form's gradients come from the pass after the step before, into
+    // the buffer of this state's parity; elsewhere a pre-pass fills the first
+    const float *gradients = kHang == 1 && !kGate && d.plan.split && parity ? d.gradients_b : d.gradients;
 
     const TilePlan &P = d.plan;
     const bool hanging = kHang == 1 || (kHang == 2 && m.hang_cells > 0);
     Tile tl;
+    const int32_t *ext, *srel;
+    const uint32_t *lohi, *fdesc;
+    const uint16_t *fidx;
     {
         const int4 *head = P.tile_head + 4 * t_index;
         const int4 h0 = head[0], h1 = head[1], h2 = head[2], h3 = head[3];
@@ -210,65 +284,56 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         tl.n_faces = h2.x;
         tl.cbase = h2.y;
         tl.sbase = h2.z;
-        tl.ext = P.ext_rel + h2.w;
-        tl.srel = P.side_rel + h3.x;
-        tl.lohi = P.side_lohi + h3.x;
-        tl.fdesc = P.face_desc + h3.y;
-        tl.fidx = P.face_idx + h3.z;
+        ext = P.ext_rel + h2.w;
+        srel = P.side_rel + h3.x;
+        lohi = P.side_lohi + h3.x;
+        fdesc = P.face_desc + h3.y;
+        fidx = P.face_idx + h3.z;
     }
-    const int E = P.max_ext;
-    // The first six arrays are dead once the depth update is done; the
-    // budget reduction then reuses their 24 * E bytes.
+    const int E = P.max_ext;   // a multiple of 4, as max_sides, so that every array starts on 16 bytes
+    // The first five arrays are dead once the depth update is done; the
+    // budget reduction then reuses their 20 * E bytes.
     float *sh_h = reinterpret_cast<float *>(smem_raw);
     float *sh_rq = sh_h + E;     // rain rate of the cell (0 when not raining)
     float *sh_area = sh_rq + E;
-    int *sh_g = reinterpret_cast<int *>(sh_area + E);
-    int *sh_bi = sh_g + E;       // boundary id, -1 for none
+    int *sh_bi = reinterpret_cast<int *>(sh_area + E);  // boundary id, -1 for none
     uint32_t *sh_fdesc = reinterpret_cast<uint32_t *>(sh_bi + E);
     float *sh_z = reinterpret_cast<float *>(sh_fdesc + E);
     float *sh_s = sh_z + E;      // donor factor, then the new depth
     float *sh_q = sh_s + E;      // q*, then final q
     float *sh_len = sh_q + P.max_sides;
-    int32_t *sh_srel = reinterpret_cast<int32_t *>(sh_len + P.max_sides);
-    uint32_t *sh_lohi = reinterpret_cast<uint32_t *>(sh_srel + P.max_sides);
+    float2 *sh_sdn = reinterpret_cast<float2 *>(sh_len + P.max_sides);  // centre distance, Manning n (stage_sdn)
+    int32_t *sh_gid = reinterpret_cast<int32_t *>(sh_sdn + (P.stage_sdn ? P.max_sides : 0));
+    uint32_t *sh_lohi = reinterpret_cast<uint32_t *>(sh_gid + P.max_sides);
     uint16_t *sh_fidx = reinterpret_cast<uint16_t *>(sh_lohi + P.max_sides);
 
-    // P0: stage the tile in two asynchronous phases. (a) The pattern's index
-    // tables (contiguous in global memory; the ring list goes to sh_g for now).
-    for (int i = tid; i < tl.n_ext; i += NT) cp_async4(sh_g + i, tl.ext + i);
-    for (int i = tid; i < tl.n_sides; i += NT) {
-        cp_async4(sh_srel + i, tl.srel + i);
-        cp_async4(sh_lohi + i, tl.lohi + i);
-    }
-    for (int i = tid; i <= tl.n_don; i += NT) cp_async4(sh_fdesc + i, tl.fdesc + i);
-    for (int i = tid; i < (tl.n_faces + 1) >> 1; i += NT)  // patterns keep an even length
-        cp_async4(reinterpret_cast<uint32_t *>(sh_fidx) + i, reinterpret_cast<const uint32_t *>(tl.fidx) + i);
-    cp_async_wait_all();
-    __syncthreads();
-    // (b) Gathers: depth and bed of the tile and its rings, the per-cell
-    // inputs of the donor rings (the rain pixel index parks in sh_rq), and q and
-    // length of every local side.
+    // P0: stage the tile in one asynchronous phase: the pattern's tables that
+    // later phases index (16 bytes at a time), and through its cell and side
+    // lists, read in place, depth and bed of the tile and its rings, the
+    // per-cell inputs of the donor rings, and q, length, centre distance and
+    // Manning n of every local side.
+    for (int i = tid; i < (tl.n_sides + 3) >> 2; i += NT)
+        cp_async16(sh_lohi + 4 * i, lohi + 4 * i);
+    for (int i = tid; i <= tl.n_don >> 2; i += NT) cp_async16(sh_fdesc + 4 * i, fdesc + 4 * i);
+    for (int i = tid; i < (tl.n_faces + 7) >> 3; i += NT) cp_async16(sh_fidx + 8 * i, fidx + 8 * i);
     for (int i = tid; i < tl.n_ext; i += NT) {
-        const int g = i ? tl.cbase + sh_g[i] : 0;
-        sh_g[i] = g;
+        const int g = i ? tl.cbase + __ldg(ext + i) : 0;
         if (i) cp_async4(sh_h + i, depth_in + g);
         else sh_h[0] = m.depth[0];
         cp_async4(sh_z + i, m.bed + g);
         if (i >= 1 && i <= tl.n_don) {
             cp_async4(sh_area + i, m.area + g);
             cp_async4(sh_bi + i, m.boundary_id + g);
-            cp_async4(sh_rq + i, m.rain_index + g);
+            cp_async4(sh_rq + i, d.rain_rate + g);
         }
     }
     for (int j = tid; j < tl.n_sides; j += NT) {
-        const int gid = tl.sbase + sh_srel[j];
+        const int gid = tl.sbase + __ldg(srel + j);
+        sh_gid[j] = gid;
         cp_async4(sh_q + j, q_in + gid);
         cp_async4(sh_len + j, m.length + gid);
+        if (P.stage_sdn) cp_async8(sh_sdn + j, d.sdn + gid);
     }
-    tl.srel = sh_srel;
-    tl.lohi = sh_lohi;
-    tl.fdesc = sh_fdesc;
-    tl.fidx = sh_fidx;
     if (tid == 0) sh_s[0] = 0.0f;  // donor_scale of the exterior sentinel (the outer ring is never a donor)
     cp_async_wait_all();
     __syncthreads();
@@ -277,42 +342,40 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     // whose flow height is below min_h gets q = +0 whatever its other inputs
     // (select then * bf), so their loads and arithmetic are skipped.
     for (int j = tid; j < tl.n_sides; j += NT) {
-        const int gid = tl.sbase + tl.srel[j];
-        const uint32_t lh = tl.lohi[j];
-        const int a = (int)(lh & 0xffffu), b = (int)(lh >> 16);
+        const uint32_t lh = sh_lohi[j];
+        const int a = (int)(lh & kSlot), b = (int)(lh >> 16);
         float zl = sh_z[a], zh = sh_z[b];
         float hl = zl + sh_h[a], hr = zh + sh_h[b];
-        float xwh = maxf(hl, hr) - maxf(maxf(zl, zh), kDh);
+        float xwh = maxf(hl, hr) - rmaxc(maxf(zl, zh), kDh);
         float new_q = 0.0f;
         if (!(xwh < d.min_h)) {
             float xq = sh_q[j];
-            const float2 sdn = d.sdn[gid];
+            const float2 sdn = P.stage_sdn ? sh_sdn[j] : d.sdn[sh_gid[j]];
             float dx = sdn.x;
             float n = sdn.y;
             // exterior sides (exactly one neighbour, the sentinel slot 0) are closed
             // (sbf, build_boundary_fdb in domain.py:472-479; checked by the planner)
             float bf = (a == 0) != (b == 0) ? 0.0f : 1.0f;
             float difference = hr - hl;
-            if (hanging) {
-                int index = m.edge_index[gid];
-                if (index >= 0 && sh_h[a] > d.min_h && sh_h[b] > d.min_h) {
-                    int axis = m.topology[3 * gid] == 2 ? 1 : 0;
-                    float o0 = m.offsets[2 * index], o1 = m.offsets[2 * index + 1];
-                    if (o0 != 0.0f) difference -= d.gradients[2 * m.slots[2 * index] + axis] * o0;
-                    if (o1 != 0.0f) difference += d.gradients[2 * m.slots[2 * index + 1] + axis] * o1;
-                }
+            if (hanging && (lh & kHangSide) && sh_h[a] > d.min_h && sh_h[b] > d.min_h) {
+                const int gid = sh_gid[j];
+                const int index = m.edge_index[gid];
+                int axis = m.topology[3 * gid] == 2 ? 1 : 0;
+                float o0 = m.offsets[2 * index], o1 = m.offsets[2 * index + 1];
+                if (o0 != 0.0f) difference -= gradients[2 * m.slots[2 * index] + axis] * o0;
+                if (o1 != 0.0f) difference += gradients[2 * m.slots[2 * index + 1] + axis] * o1;
             }
-            float xdq = (d.neg_g * difference / dx) * maxf(xwh, 0.0f) * dt;
+            float xdq = (d.neg_g * difference / dx) * rmaxc(xwh, 0.0f) * dt;
             float ratio = 0.0f;
-            if (xq != 0.0f) ratio = xq / pow_real(maxf(xwh, 0.00001f), d.seven_thirds);
+            if (xq != 0.0f) ratio = xq / pow_real(rmaxc(xwh, 0.00001f), d.seven_thirds);
             float xf = 1.0f + d.g * dt * (n * n) * fabsf(ratio);
             float nb;
             if (kThetaOne) {
                 nb = 0.0f + 0.0f;
             } else {
-                int so = m.topology[3 * gid];
+                int so = m.topology[3 * sh_gid[j]];
                 int dl = so == 2 ? 0 : 2, dr = so == 2 ? 1 : 3;
-                int ga = sh_g[a], gb = sh_g[b];
+                int ga = a ? tl.cbase + __ldg(ext + a) : 0, gb = b ? tl.cbase + __ldg(ext + b) : 0;
                 nb = boundary_neighbor_sum(xq, d.face_qn[4 * ga + dl], d.face_qn[4 * gb + dr],
                                            m.open_face[4 * ga + dl], m.open_face[4 * gb + dr]);
             }
@@ -333,28 +396,15 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             float discharge = 0.0f;
             if (bi >= 0) {
                 kind = m.kind[bi];
-                if (kind == 1) discharge = d.values[bi] * m.weight[sh_g[i]];
+                if (kind == 1) discharge = d.values[bi] * m.weight[tl.cbase + __ldg(ext + i)];
             }
-            // rain rate from the staged pixel index, kept for the depth update
-            const float rainq = raining ? d.rain_rates[__float_as_int(sh_rq[i])] : 0.0f;
-            sh_rq[i] = rainq;
+            const float rainq = sh_rq[i];
             float pipe = 0.0f;
-            float positive = (maxf(pipe, 0.0f) + maxf(discharge, 0.0f)) * dt;
+            float positive = (rmaxc(pipe, 0.0f) + rmaxc(discharge, 0.0f)) * dt;
             float area = sh_area[i];
             float available = sh_h[i] * area + positive + rainq * dt * area;
-            float outgoing = (maxf(-pipe, 0.0f) + maxf(-discharge, 0.0f)) * dt;
-            uint32_t fd = tl.fdesc[i];
-            int k = (int)(fd & 0xffffu);
-            uint32_t counts = fd >> 16;
-            for (int dd = 0; dd < 4; ++dd) {
-                int cntd = (int)((counts >> (4 * dd)) & 15u);
-                for (int jj = 0; jj < cntd; ++jj) {
-                    int ls = tl.fidx[k++];
-                    float signed_q = sh_q[ls] * sh_len[ls];
-                    if (dd == 0 || dd == 2) signed_q = -signed_q;
-                    outgoing += maxf(signed_q, 0.0f) * dt;
-                }
-            }
+            float outgoing = (rmaxc(-pipe, 0.0f) + rmaxc(-discharge, 0.0f)) * dt;
+            outgoing = face_outflow(sh_fdesc[i], sh_fidx, sh_q, sh_len, dt, outgoing);
             float sc = 1.0f;
             if (outgoing > available && kind != 0) {
                 sc = available / outgoing;
@@ -378,8 +428,8 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     {
         uint32_t my_faces = 0;
         for (int j = tid; j < tl.n_qf; j += NT) {
-            const uint32_t lh = tl.lohi[j];
-            const int a = (int)(lh & 0xffffu), b = (int)(lh >> 16);
+            const uint32_t lh = sh_lohi[j];
+            const int a = (int)(lh & kSlot), b = (int)(lh >> 16);
             float q = sh_q[j];
             int donor = q >= 0.0f ? a : b;
             float sc = sh_s[donor];
@@ -443,7 +493,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         float discharge = 0.0f;
         if (kind == 1) {
             float requested = d.values[bi] * in_w[kk];
-            discharge = maxf(requested, 0.0f) + minf(requested, 0.0f) * sc;
+            discharge = rmaxc(requested, 0.0f) + minf(requested, 0.0f) * sc;
             terms.discharge[kk] = discharge * dt;
         }
         float ssq = pipe + discharge;
@@ -460,7 +510,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             infil = in_inf[kk];
         }
         float fl[4];
-        face_sums(tl, sh_q, sh_len, slot, fl);
+        face_sums(sh_fdesc[slot], sh_fidx, sh_q, sh_len, fl);
         float ql = fl[0], qr = fl[1], qb = fl[2], qt = fl[3];
         float tq = ql - qr + qb - qt + ssq;
         float ea = sh_area[slot];
@@ -470,14 +520,14 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         float increment = (flux == 0.0f ? flux : flux / ea) + rain_depth;
         float previous = sh_h[slot];
         float raw_depth = previous + increment;
-        float removed = minf(infil * dt, maxf(raw_depth, 0.0f));
+        float removed = minf(infil * dt, rmaxc(raw_depth, 0.0f));
         raw_depth -= removed;
-        float floor_v = maxf(-raw_depth, 0.0f);
+        float floor_v = rmaxc(-raw_depth, 0.0f);
         terms.removed[kk] = removed * ea;
         terms.floor_v[kk] = floor_v * ea;
         float depth;
         if (kind == 0) {
-            float target = maxf(d.level_values[bi] - sh_z[slot], 0.0f);
+            float target = rmaxc(d.level_values[bi] - sh_z[slot], 0.0f);
             terms.level[kk][0] = (target - previous) * ea;
             terms.level[kk][1] = -(ql - qr + qb - qt) * dt;
             terms.level[kk][2] = -pipe * dt;
@@ -485,12 +535,12 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             terms.level[kk][4] = removed * ea;
             depth = target;
         } else {
-            depth = maxf(raw_depth, 0.0f);
+            depth = rmaxc(raw_depth, 0.0f);
         }
         depth_out[g] = depth;
         sh_s[slot] = depth;
         const float fastest = fastest_speed(depth >= d.min_h, ql + qr, qb + qt, in_hgt[kk], in_wid[kk],
-                                            maxf(depth, 0.01f), in_ms[kk]);
+                                            rmaxc(depth, 0.01f), in_ms[kk]);
         if (fastest > in_ms[kk]) m.max_speed[g] = fastest;
         if (depth > in_md[kk]) {
             m.max_depth[g] = depth;
@@ -531,7 +581,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     }
     // ring 1 (fused-CFL form): the new depth only, for the CFL of owned sides
     for (int i = tl.n_r0 + 1 + tid; i <= tl.n_r01; i += NT) {
-        const int g = sh_g[i];
+        const int g = tl.cbase + __ldg(ext + i);
         const int bi = sh_bi[i];
         const int kind = bi >= 0 ? m.kind[bi] : -1;
         float sc = sh_s[i];
@@ -540,7 +590,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         float discharge = 0.0f;
         if (kind == 1) {
             float requested = d.values[bi] * m.weight[g];
-            discharge = maxf(requested, 0.0f) + minf(requested, 0.0f) * sc;
+            discharge = rmaxc(requested, 0.0f) + minf(requested, 0.0f) * sc;
         }
         float ssq = pipe + discharge;
         float rainq = sh_rq[i];
@@ -554,16 +604,16 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             infil = m.infiltration[g];
         }
         float fl[4];
-        face_sums(tl, sh_q, sh_len, i, fl);
+        face_sums(sh_fdesc[i], sh_fidx, sh_q, sh_len, fl);
         float tq = fl[0] - fl[1] + fl[2] - fl[3] + ssq;
         float ea = sh_area[i];
         float rain_depth = rainq * dt;
         float flux = tq * dt;
         float increment = (flux == 0.0f ? flux : flux / ea) + rain_depth;
         float raw_depth = sh_h[i] + increment;
-        float removed = minf(infil * dt, maxf(raw_depth, 0.0f));
+        float removed = minf(infil * dt, rmaxc(raw_depth, 0.0f));
         raw_depth -= removed;
-        float depth = kind == 0 ? maxf(d.level_values[bi] - sh_z[i], 0.0f) : maxf(raw_depth, 0.0f);
+        float depth = kind == 0 ? rmaxc(d.level_values[bi] - sh_z[i], 0.0f) : rmaxc(raw_depth, 0.0f);
         sh_s[i] = depth;
     }
     __syncthreads();
@@ -577,7 +627,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     // and a shuffle tree does strides 16 .. 1.
     if (T <= 32) {
         double *buf = reinterpret_cast<double *>(smem_raw);
-        const int cap = (24 * E) / (NT * 8);  // >= 1: the planner pads E
+        const int cap = (20 * E) / (NT * 8);  // >= 1: the planner pads E
         const int lane_b = tid & 31, warp_b = tid >> 5;
 #pragma unroll
         for (int kk = 0; kk < CPT; ++kk) {
@@ -628,7 +678,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
                 float val = term_value(t, B, terms.removed[kk], terms.floor_v[kk], terms.level[kk],
                                        terms.discharge[kk], terms.bi[kk], terms.kind[kk]);
                 if (!__syncthreads_or(val != 0.0f)) continue;
-                // the tree's NT doubles live in the dead shared arrays (24 * E >= 8 * NT)
+                // the tree's NT doubles live in the dead shared arrays (20 * E >= 8 * NT)
                 double sum = tree_halves<NT>((double)val, reinterpret_cast<double *>(smem_raw));
                 const int blk = blk0 + (tid >> 8);
                 if ((tid & 255) == 0 && blk < d.blocks && sum != 0.0)
@@ -658,32 +708,37 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         }
     }
 
-    // P5: owned sides: final q out; in the fused-CFL form also the CFL of the
-    // owned sides with the new depths (the split form's CFL pass follows).
+    // P5: owned sides: final q out, and the CFL on the new depths: of every
+    // owned side in the fused-CFL form; in the split form of those whose two
+    // cells are the tile's (the edge pass takes the others), unless a full CFL
+    // pass follows (ensemble launches; gate runs, which move beds first). Starting
+    // from the minimum of the blocks that are done spares 4 % of the instructions
+    // but its hot word costs more (1.36 M cells: 4538 to 4661 us per 32 steps).
     const bool split = P.split != 0;
+    const int last_cell = !split ? tl.n_ext : (kGate || kHang == 2) ? 0 : tl.n_r0;
     unsigned long long best = kCflEmpty;
     for (int j = tid; j < tl.n_owned; j += NT) {
-        const int gid = tl.sbase + tl.srel[j];
+        const int gid = sh_gid[j];
         float qv = sh_q[j];
         q_out[gid] = qv;
-        if (split) continue;
-        const uint32_t lh = tl.lohi[j];
-        const int a = (int)(lh & 0xffffu), b = (int)(lh >> 16);
-        if (a != 0 && b != 0) {
+        if (kGate) continue;
+        const uint32_t lh = sh_lohi[j];
+        const int a = (int)(lh & kSlot), b = (int)(lh >> 16);
+        if (a != 0 && b != 0 && a <= last_cell && b <= last_cell) {
             float zl = sh_z[a], zh = sh_z[b];
             float head = maxf(zl + sh_s[a], zh + sh_s[b]);
-            float h = maxf(head - maxf(maxf(zl, zh), kDh), 0.01f);
+            float h = rmaxc(head - rmaxc(maxf(zl, zh), kDh), 0.01f);
             fold_cfl(d, sh_len[j], qv, h, (unsigned)gid, best);
         }
     }
-    if (!split) {
-        best = warp_min_u64(best);
+    if (last_cell) {
+        best = warp_min_key(best);
         if ((tid & 31) == 0) sh_min[tid >> 5] = best;
     }
     if (my_wet) atomicAdd(&sh_cnt[2], my_wet);
     __syncthreads();
     if (tid == 0) {
-        if (!split) {
+        if (last_cell) {
             unsigned long long bmin = kCflEmpty;
             for (int w = 0; w < NT / 32; ++w) bmin = sh_min[w] < bmin ? sh_min[w] : bmin;
             if (bmin != kCflEmpty) atomicMin(&c->cfl_packed, bmin);
@@ -705,25 +760,20 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     __threadfence();
     c->done_blocks = 0;
     if (!split) {
-        unsigned long long packed = atomicExch(&c->cfl_packed, kCflEmpty);
-        if (packed == kCflEmpty) {
-            c->ndt = __uint_as_float(0x7f800000u);
-            c->cfl_arg = 0;
-        } else {
-            c->ndt = __uint_as_float((uint32_t)(packed >> 32));
-            c->cfl_arg = (int32_t)(packed & 0xffffffffu);
-        }
+        set_cfl(c);
     }
     finish_step(c);
+    c->grad_parity = gradients == d.gradients ? 0 : 1;
     c->parity = parity ^ 1;
     if (!split && c->slot < d.batch_size) prepare_step(d, c, depth_out, q_out);
 }
 
-// CFL pass (solver_compact.py:617-641) over sides [first, end) with stride,
-// on the current (just updated) state; each block adds its minimum packed
-// key (cfl bits, side id) and the last of `blocks` blocks sets ndt /
-// cfl_arg (the lowest side id attains the minimum) and prepares the next
-// step (solver_compact.py:364-382).
+// CFL pass (solver_compact.py:617-641) over sides [first, end) with stride (or,
+// kEdges, over the plan's sides between tiles), on the current (just updated)
+// state; each block adds its minimum packed key (cfl bits, side id) and the
+// last of `blocks` blocks sets ndt / cfl_arg (the lowest side id attains the
+// minimum) and prepares the next step (solver_compact.py:364-382).
+template <bool kEdges = false>
 __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int stride, unsigned blocks,
                                          const GateDev *gd = nullptr)
 {
@@ -735,14 +785,21 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
     const int active = c->active;
     const float *depth = cur_depth(d, c->parity);
     const float *q = cur_q(d, c->parity);
-    unsigned long long best = kCflEmpty;
+    // sides between tiles start from the minimum of those inside
+    unsigned long long best = kEdges ? __ldcg(&c->cfl_packed) : kCflEmpty;
     if (active) {
-        for (int si = first + (int)threadIdx.x; si < end; si += stride) {
-            const int el = m.topology[3 * si + 1], eh = m.topology[3 * si + 2];
-            if (el != 0 && eh != 0) {
+        for (int i = first + (int)threadIdx.x; i < end; i += stride) {
+            int si = i, el, eh;
+            if (kEdges) {
+                const int4 edge = d.plan.edges[i];
+                el = edge.x; eh = edge.y; si = edge.z;
+            } else {
+                el = m.topology[3 * si + 1]; eh = m.topology[3 * si + 2];
+            }
+            if (kEdges || (el != 0 && eh != 0)) {
                 const float zl = m.bed[el], zh = m.bed[eh];
                 const float head = maxf(zl + depth[el], zh + depth[eh]);
-                const float h = maxf(head - maxf(maxf(zl, zh), kDh), 0.01f);
+                const float h = rmaxc(head - rmaxc(maxf(zl, zh), kDh), 0.01f);
                 fold_cfl(d, m.length[si], q[si], h, (unsigned)si, best);
             }
         }
@@ -765,17 +822,8 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
     if (!last) return;
     if (threadIdx.x == 0) {
         __threadfence();
-        const unsigned long long packed = atomicExch(&c->cfl_packed, kCflEmpty);
         c->done_blocks = 0;
-        if (active) {
-            if (packed == kCflEmpty) {
-                c->ndt = __uint_as_float(0x7f800000u);
-                c->cfl_arg = 0;
-            } else {
-                c->ndt = __uint_as_float((uint32_t)(packed >> 32));
-                c->cfl_arg = (int32_t)(packed & 0xffffffffu);
-            }
-        }
+        if (active) set_cfl(c);
         prepared = c->slot < d.batch_size;
         if (prepared) prepare_step(d, c, depth, q);
     }
@@ -806,12 +854,28 @@ __global__ void __launch_bounds__(256, 4) k_step_tiled_gate(const __grid_constan
     step_tile<kThetaOne, kHanging ? 1 : 0, 256, 1, true>(d, blockIdx.x, gridDim.x, &g);
 }
 
-// CFL pass of one mesh after its fused step (grid-stride over the sides);
-// split plans only.
-__global__ void __launch_bounds__(256) k_cfl_tiled(const __grid_constant__ Dev d)
+// After the fused step of a split plan: the CFL of the sides between tiles and,
+// in the blocks beyond those, the next step's hanging-edge gradients (which
+// depend on the new depths only) into the buffer of the new state's parity.
+// Both wait on memory, so one launch hides them behind each other. On the
+// quadtree of 1.36 M cells a full CFL pass took 23 us and the gradient pre-pass 8
+// (cold) per step; 232 thousand of its 2.73 M sides lie between tiles. With the
+// staging in one phase, 32 steps: 4878 to 4535 us.
+__global__ void __launch_bounds__(256) k_edges_tiled(const __grid_constant__ Dev d, unsigned cfl_blocks)
 {
-    if (!d.plan.split) return;
-    cfl_pass(d, 1 + (int)(blockIdx.x * blockDim.x), d.m.s_num, (int)(gridDim.x * blockDim.x), gridDim.x);
+    if (blockIdx.x >= cfl_blocks) {
+        const int i = (int)((blockIdx.x - cfl_blocks) * blockDim.x + threadIdx.x);
+        const Ctl *c = d.ctl;
+        // the other blocks' last one prepares the next step meanwhile; where that
+        // will do nothing (or this step did), no gradients are needed, and
+        // parity does not change before the next step
+        if (!c->active) return;
+        const int parity = c->parity;
+        if (i < 2 * d.m.hang_cells && d.hang[i].cell != -1)
+            (parity ? d.gradients_b : d.gradients)[i] = hang_gradient(d, cur_depth(d, parity), i >> 1, i & 1);
+        return;
+    }
+    cfl_pass<true>(d, (int)(blockIdx.x * blockDim.x), d.plan.n_edges, (int)(cfl_blocks * blockDim.x), cfl_blocks);
 }
 
 // CFL pass of a gate run (split plan): also the next step's check_gates.
@@ -839,12 +903,19 @@ __global__ void __launch_bounds__(NT, kEnsembleMinBlocks<NT>)
 }
 
 // Batch start: the rain-time second buffer equals the caller's buffer (cells
-// that do not rain during the batch are never rewritten).
+// that do not rain during the batch are never rewritten); every cell's rain
+// rate, fixed during a batch.
+__device__ __forceinline__ void start_cell(const Dev &d, int i)
+{
+    d.rain_time_b[i] = d.m.rain_time[i];
+    d.rain_rate[i] = i && d.ctl->raining ? d.rain_rates[d.m.rain_index[i]] : 0.0f;
+}
+
 __global__ void k_batch_start(Dev d)
 {
     const nhf_mesh &m = d.m;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.e_num; i += gridDim.x * blockDim.x)
-        d.rain_time_b[i] = m.rain_time[i];
+        start_cell(d, i);
 }
 
 // Batch end: bring the current state back into the caller's buffers.
@@ -947,7 +1018,7 @@ struct HostMesh {
     int e, s;
     std::vector<int32_t> topo, fptr, fcnt, isl;
     std::vector<uint8_t> sbf;
-    std::vector<int32_t> edge;  // hanging edge of each side (resident plans of meshes with hanging edges)
+    std::vector<int32_t> edge;  // hanging edge of each side (meshes with hanging edges)
 };
 
 int copy_back(const nhf_mesh &m, cudaStream_t st, HostMesh &hm)
@@ -997,7 +1068,7 @@ bool consistent(const HostMesh &hm, std::string &why)
 
 int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::vector<int32_t> &tile_pattern,
                std::vector<int32_t> &tile_cbase, std::vector<int32_t> &tile_sbase, int &max_ext, int &max_sides,
-               int &max_faces, int rings, std::string &why, ResidentArgs *resident)
+               int &max_faces, int rings, std::string &why, ResidentArgs *resident, std::vector<int4> *edges)
 {
     const int e = hm.e, s = hm.s;
     // cell adjacency through interior sides
@@ -1024,6 +1095,7 @@ int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::v
     tile_cbase.assign(n_tiles, 0);
     tile_sbase.assign(n_tiles, 0);
     max_ext = max_sides = max_faces = 0;
+    if (edges) edges->clear();
     std::vector<int> ext, sides;
     for (int t = 0; t < n_tiles; ++t) {
         const int cbase = t * T;
@@ -1083,7 +1155,7 @@ int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::v
             n_owned += (sflag[sides[i]] & kOwned) ? 1 : 0;
             n_qf += (sflag[sides[i]] & (kOwned | kFinal)) ? 1 : 0;
         }
-        if ((int)ext.size() > 65535 || (int)sides.size() > 65535) { why = "tile halo too large"; return 1; }
+        if ((int)ext.size() > (int)kSlot || (int)sides.size() > 65535) { why = "tile halo too large"; return 1; }
         int sbase = sides.empty() ? 0 : *std::min_element(sides.begin(), sides.end());
         Pattern p;
         p.counts = {(int)ext.size(), n_r0, n_r01, n_don, (int)sides.size(), n_owned, n_qf, r0_first - cbase,
@@ -1098,10 +1170,17 @@ int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::v
             p.srel[i] = sid - sbase;
             int lo = hm.topo[3 * sid + 1], hi = hm.topo[3 * sid + 2];
             p.lohi[i] = (uint32_t)slot[lo] | ((uint32_t)slot[hi] << 16);
+            if (!resident && !hm.edge.empty() && hm.edge[sid] >= 0) p.lohi[i] |= kHangSide;
         }
+        if (edges)
+            for (int i = 0; i < n_owned; ++i) {
+                const int sid = sides[i], lo = hm.topo[3 * sid + 1], hi = hm.topo[3 * sid + 2];
+                if (lo && hi && (ring[lo] != 0 || ring[hi] != 0)) edges->push_back(make_int4(lo, hi, sid, 0));
+            }
         p.fdesc.assign(n_don + 1, 0u);
         for (int i = 1; i <= n_don; ++i) {
             int cc = ext[i];
+            while (p.fidx.size() & 3) p.fidx.push_back(0);  // a cell's list starts on 8 bytes
             if (p.fidx.size() > 65535) { why = "tile face table too large"; return 1; }
             uint32_t counts = 0;
             uint32_t start = (uint32_t)p.fidx.size();
@@ -1231,7 +1310,7 @@ __global__ void k_ens_batch_start(const Dev *devs, const int2 *items)
     const int2 w = items[blockIdx.x];
     const Dev &d = devs[w.x];
     const int end = min(d.m.e_num, (w.y + 1) * kEnsChunk);
-    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x) d.rain_time_b[i] = d.m.rain_time[i];
+    for (int i = w.y * kEnsChunk + threadIdx.x; i < end; i += blockDim.x) start_cell(d, i);
 }
 
 __global__ void k_ens_pressure(const Dev *devs, const int2 *items)
@@ -1315,7 +1394,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     HostMesh hm;
     if (copy_back(m, s, hm)) return bad("copying the mesh tables to the host failed");
     if (!consistent(hm, reason)) return bad(reason);
-    if (resident && m.hang_cells > 0) {
+    if (m.hang_cells > 0) {
         hm.edge.resize((size_t)m.s_num);
         if (cudaMemcpyAsync(hm.edge.data(), m.edge_index, 4 * hm.edge.size(), cudaMemcpyDeviceToHost, s) ||
             cudaStreamSynchronize(s))
@@ -1323,6 +1402,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     }
     std::vector<Pattern> patterns;
     std::vector<int32_t> tp, tc, ts;
+    std::vector<int4> edges;   // split plans: the sides between tiles
     int max_ext = 0, max_sides = 0, max_faces = 0, tile = 0;
     size_t smem = 0;
     // Small meshes take small tiles so that every SM gets work.
@@ -1337,23 +1417,36 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
             return bad("tile size must be 256, 512 or 1024");
         sizes = {tile_request};
     }
-    bool split = false;
+    bool split = false, stage_sdn = true;
     for (int T : sizes) {
         // The separate CFL pass pays one launch per step for less halo work
         // (no ring 3, no ring-1 depth recompute): worth it from two waves of
-        // resident blocks on.
+        // resident blocks on, and wherever there are hanging edges, whose
+        // gradients take a launch in either form (32 steps of 0.19 M cells 1263
+        // to 1016 us, of six members of 1.2 M cells together 5067 to 4235).
         const int wave = 148 * (T == 256 ? kMinBlocks<256> : kMinBlocks<512>);
         const int n_tiles = (m.e_num + T - 1) / T;
-        split = cfl_mode == 2 || (cfl_mode == 0 && n_tiles >= 2 * wave);
+        split = cfl_mode == 2 || (cfl_mode == 0 && (n_tiles >= 2 * wave || m.hang_cells > 0));
         if (plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason,
-                       resident))
+                       resident, split ? &edges : nullptr))
             return bad(reason);
         // The budget reduction stages one term of every thread (NT doubles)
-        // in the 24 * max_ext bytes of shared arrays that are dead after the
+        // in the 20 * max_ext bytes of shared arrays that are dead after the
         // depth update; meshes smaller than a tile need the padding.
         const int nt = T == 256 ? 256 : 512;
-        if (24 * max_ext < 8 * nt) max_ext = (8 * nt + 23) / 24;
-        smem = (size_t)max_ext * 32 + (size_t)max_sides * 16 + (size_t)max_faces * 2 + 16;
+        if (20 * max_ext < 8 * nt) max_ext = (8 * nt + 19) / 20;
+        max_ext = (max_ext + 3) & ~3;   // every array of a tile starts on 16 bytes
+        max_sides = (max_sides + 3) & ~3;
+        // centre distance and Manning n are staged with the tile where that
+        // costs no resident block (members of 0.1 to 0.2 M cells with four
+        // blocks per SM instead of five ran 5 % slower)
+        const size_t lean = (size_t)max_ext * 28 + (size_t)max_sides * 16 + (size_t)((max_faces + 7) & ~7) * 2 + 16;
+        auto resident_blocks = [&](size_t bytes) {
+            return std::min(T == 256 ? kMinBlocks<256> : kMinBlocks<512>, (int)(228 * 1024 / (bytes + 1024 + 256)));
+        };
+        smem = lean + (size_t)max_sides * 8;
+        stage_sdn = smem <= (size_t)kMaxSharedBytes && resident_blocks(smem) == resident_blocks(lean);
+        if (!stage_sdn) smem = lean;
         if (resident || smem <= (size_t)kMaxSharedBytes) { tile = T; break; }
     }
     if (!tile) return bad("tile halos exceed shared memory (cell numbering is not spatially coherent)");
@@ -1372,9 +1465,13 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         lohi.insert(lohi.end(), p.lohi.begin(), p.lohi.end());
         fdesc.insert(fdesc.end(), p.fdesc.begin(), p.fdesc.end());
         fidx.insert(fidx.end(), p.fidx.begin(), p.fidx.end());
-        if (fidx.size() & 1) fidx.push_back(0);  // the kernel copies face indices in pairs
+        // the kernels copy the tables 16 bytes at a time
+        while (ext.size() & 3) ext.push_back(0);
+        while (srel.size() & 3) { srel.push_back(0); lohi.push_back(0); }
+        while (fdesc.size() & 3) fdesc.push_back(0);
+        while (fidx.size() & 7) fidx.push_back(0);
     }
-    if (fidx.empty()) { fidx.push_back(0); fidx.push_back(0); }
+    while (fidx.size() < 8) fidx.push_back(0);
     // per-tile header: the pattern's counts and offsets with the tile's bases
     std::vector<int32_t> head((size_t)tp.size() * 16, 0);
     for (size_t t = 0; t < tp.size(); ++t) {
@@ -1385,13 +1482,15 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         h[9] = tc[t]; h[10] = ts[t];
         h[11] = off[0]; h[12] = off[1]; h[13] = off[2]; h[14] = off[3];
     }
-    if (srel.empty()) { srel.push_back(0); lohi.push_back(0); }
+    while (srel.size() < 4) { srel.push_back(0); lohi.push_back(0); }
+    if (edges.empty()) edges.push_back(make_int4(0, 0, 0, 0));
+    const int n_edges = split ? (int)edges.size() : 0;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
     size_t o_ext = take(ext.size() * 4);
     size_t o_srel = take(srel.size() * 4), o_lohi = take(lohi.size() * 4), o_fd = take(fdesc.size() * 4);
     size_t o_fi = take(fidx.size() * 2);
-    size_t o_hd = take(head.size() * 4);
+    size_t o_hd = take(head.size() * 4), o_ed = take(edges.size() * sizeof(int4));
     void *mem = nullptr;
     if (cudaMalloc(&mem, off) != cudaSuccess) return bad("allocating the tile plan failed");
     char *b = (char *)mem;
@@ -1401,7 +1500,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     bool ok = up(o_ext, ext.data(), ext.size() * 4) &&
               up(o_srel, srel.data(), srel.size() * 4) && up(o_lohi, lohi.data(), lohi.size() * 4) &&
               up(o_fd, fdesc.data(), fdesc.size() * 4) && up(o_fi, fidx.data(), fidx.size() * 2) &&
-              up(o_hd, head.data(), head.size() * 4) &&
+              up(o_hd, head.data(), head.size() * 4) && up(o_ed, edges.data(), edges.size() * sizeof(int4)) &&
               cudaStreamSynchronize(s) == cudaSuccess;
     if (!ok) { cudaFree(mem); return bad("uploading the tile plan failed"); }
     TilePlan &P = out->plan;
@@ -1412,6 +1511,9 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     P.cells_per_thread = tile == 1024 ? 2 : 1;
     P.split = split ? 1 : 0;
     P.tile_head = (const int4 *)(b + o_hd);
+    P.edges = (const int4 *)(b + o_ed);
+    P.n_edges = n_edges;
+    P.stage_sdn = stage_sdn ? 1 : 0;
     P.ext_rel = (const int32_t *)(b + o_ext);
     P.side_rel = (const int32_t *)(b + o_srel);
     P.side_lohi = (const uint32_t *)(b + o_lohi);
@@ -1427,10 +1529,11 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     return 0;
 }
 
-void tiled_enqueue_step(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate)
+void tiled_enqueue_step(const Dev &d, const TiledBuild &b, int step, cudaStream_t s, const GateDev *gate)
 {
     const nhf_mesh &m = d.m;
-    if (m.hang_cells > 0) k_pressure_tiled<<<(m.hang_cells + 63) / 64, 64, 0, s>>>(d);
+    // split plans: the pass after a step leaves the next step's gradients
+    if (m.hang_cells > 0 && (step == 0 || gate || !b.plan.split)) k_pressure_tiled<<<(m.hang_cells + 63) / 64, 64, 0, s>>>(d);
     if (!d.theta_one) k_face_qn_tiled<<<(m.e_num + 255) / 256, 256, 0, s>>>(d);
     if (gate) {  // 256-cell tiles, split plan (checked when the controller is attached)
         const int grid = d.plan.n_tiles;
@@ -1456,10 +1559,12 @@ void tiled_enqueue_step(const Dev &d, const TiledBuild &b, cudaStream_t s, const
 void tiled_enqueue_cfl(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate)
 {
     if (b.plan.split) {
-        int gc = (d.m.s_num + 255) / 256;
+        const int sides = gate ? d.m.s_num : b.plan.n_edges;
+        int gc = (sides + 255) / 256;
         if (gc > 148 * 8) gc = 148 * 8;
+        if (gc < 1) gc = 1;
         if (gate) k_cfl_tiled_gate<<<gc, 256, 0, s>>>(d, *gate);
-        else k_cfl_tiled<<<gc, 256, 0, s>>>(d);
+        else k_edges_tiled<<<gc + (2 * d.m.hang_cells + 255) / 256, 256, 0, s>>>(d, (unsigned)gc);
     }
 }
 
