@@ -142,6 +142,8 @@ struct GateDev {
     int32_t *commanded, *flow_seen, *opened;
     uint32_t *command, *first_flow, *opened_at;
     double *acc_sum, *acc_comp;
+    int32_t n_edges;    // fused step: the sides inside tiles that touch a gate cell
+    const int4 *edges;  // [n_edges] lower cell, higher cell, side, 0
 };
 
 struct Dev {

@@ -35,6 +35,7 @@ struct nhf_handle {
     nhf::GateDev gate{};
     bool gate_on = false;
     void *gate_mem = nullptr;   // gate budget partials
+    void *gate_edges = nullptr; // sides of gate cells inside tiles (fused step)
     double *h_gacc = nullptr;   // pinned staging of the gate partials
     bool tiled = false;
     std::string path = "multipass";

@@ -14,8 +14,7 @@
 // step takes the CFL of the sides inside its tile and a pass after it
 // (k_edges_tiled) that of the sides between tiles, with the next step's
 // hanging-edge gradients. The halo work saved outweighs the launch
-// (TilePlan::split). Gate runs, which move beds in between, and ensemble
-// launches keep a pass over all sides.
+// (TilePlan::split). Ensemble launches keep a pass over all sides.
 // Every quantity is computed with the reference's operation order, so a cell
 // that several tiles recompute gets the same bits everywhere; each output
 // (depth, side q, extrema, budget block) has exactly one writer, its owner
@@ -45,10 +44,13 @@ namespace nhf {
 namespace {
 
 constexpr int kMaxSharedBytes = 108 * 1024;   // two blocks per SM
-// Resident blocks per SM the register budget is sized for: 5 x 256 threads
-// (48 registers) for 256-cell tiles, 2 x 512 threads (64) for larger ones.
+// Resident blocks per SM the register budget is sized for: 6 x 256 threads
+// (40 registers, 8 bytes of spills) for 256-cell tiles, 2 x 512 threads (64) for
+// larger ones. A tile's life is a chain of memory latencies and barriers, so
+// residency counts: 1.36 M cell quadtree, us per 32 steps with 4, 5, 6, 7 blocks
+// 4669, 4408, 4172, 4806.
 template <int NT>
-constexpr int kMinBlocks = NT == 256 ? 5 : 2;
+constexpr int kMinBlocks = NT == 256 ? 6 : 2;
 // The ensemble step reads its descriptor from shared memory and needs more
 // registers: 4 x 256 or 2 x 512 threads (64 registers).
 template <int NT>
@@ -236,12 +238,14 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     __shared__ uint32_t sh_minbits;
     __shared__ uint32_t sh_mask[CPT][NT / 256];
     __shared__ int sh_last;
+    __shared__ uint32_t sh_gate[kGate ? 8 : 1];  // a bit per gate cell of the tile
     Ctl *c = d.ctl;
     const nhf_mesh &m = d.m;
     const int tid = threadIdx.x;
 
     if (tid == 0) { sh_cnt[0] = sh_cnt[1] = sh_cnt[2] = 0u; sh_minbits = __float_as_uint(1.0f); }
     if (tid < CPT * (NT / 256)) (&sh_mask[0][0])[tid] = 0u;
+    if (kGate && tid < 8) sh_gate[tid] = 0u;
     const int active = c->active;
     if (!active) {
         // No physics this slot: the last block advances the slot and prepares the next.
@@ -551,6 +555,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             // record_cell, measure_inventory and the rounding term
             // (solver_compact.py:595-604; gate.py:151-193)
             const int cg = gd->cell_gate[g];
+            if (cg >= 0) atomicOr(&sh_gate[(slot - 1) >> 5], 1u << ((slot - 1) & 31));
             g_off = gd->pond[g] == 1 ? 4 * gd->count + 2 : (cg >= 0 ? 4 * gd->count + 8 + 6 * cg : -1);
             if (g_off >= 0) {
                 float applied_floor = floor_v, level_exchange = 0.0f;
@@ -710,21 +715,23 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
 
     // P5: owned sides: final q out, and the CFL on the new depths: of every
     // owned side in the fused-CFL form; in the split form of those whose two
-    // cells are the tile's (the edge pass takes the others), unless a full CFL
-    // pass follows (ensemble launches; gate runs, which move beds first). Starting
+    // cells are the tile's (the edge pass takes the others, and those of gate
+    // cells, whose beds move first), unless a full CFL pass follows (ensemble
+    // launches). Starting
     // from the minimum of the blocks that are done spares 4 % of the instructions
     // but its hot word costs more (1.36 M cells: 4538 to 4661 us per 32 steps).
     const bool split = P.split != 0;
-    const int last_cell = !split ? tl.n_ext : (kGate || kHang == 2) ? 0 : tl.n_r0;
+    const int last_cell = !split ? tl.n_ext : kHang == 2 ? 0 : tl.n_r0;
     unsigned long long best = kCflEmpty;
     for (int j = tid; j < tl.n_owned; j += NT) {
         const int gid = sh_gid[j];
         float qv = sh_q[j];
         q_out[gid] = qv;
-        if (kGate) continue;
         const uint32_t lh = sh_lohi[j];
         const int a = (int)(lh & kSlot), b = (int)(lh >> 16);
         if (a != 0 && b != 0 && a <= last_cell && b <= last_cell) {
+            if (kGate && (((sh_gate[(a - 1) >> 5] >> ((a - 1) & 31)) | (sh_gate[(b - 1) >> 5] >> ((b - 1) & 31))) & 1u))
+                continue;
             float zl = sh_z[a], zh = sh_z[b];
             float head = maxf(zl + sh_s[a], zh + sh_s[b]);
             float h = rmaxc(head - rmaxc(maxf(zl, zh), kDh), 0.01f);
@@ -791,7 +798,7 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
         for (int i = first + (int)threadIdx.x; i < end; i += stride) {
             int si = i, el, eh;
             if (kEdges) {
-                const int4 edge = d.plan.edges[i];
+                const int4 edge = i < d.plan.n_edges ? d.plan.edges[i] : gd->edges[i - d.plan.n_edges];
                 el = edge.x; eh = edge.y; si = edge.z;
             } else {
                 el = m.topology[3 * si + 1]; eh = m.topology[3 * si + 2];
@@ -878,10 +885,12 @@ __global__ void __launch_bounds__(256) k_edges_tiled(const __grid_constant__ Dev
     cfl_pass<true>(d, (int)(blockIdx.x * blockDim.x), d.plan.n_edges, (int)(cfl_blocks * blockDim.x), cfl_blocks);
 }
 
-// CFL pass of a gate run (split plan): also the next step's check_gates.
+// The same CFL pass of a gate run (split plan), after the beds have moved: the
+// sides between tiles and those of gate cells; also the next step's check_gates.
 __global__ void __launch_bounds__(256) k_cfl_tiled_gate(const __grid_constant__ Dev d, const __grid_constant__ GateDev g)
 {
-    cfl_pass(d, 1 + (int)(blockIdx.x * blockDim.x), d.m.s_num, (int)(gridDim.x * blockDim.x), gridDim.x, &g);
+    cfl_pass<true>(d, (int)(blockIdx.x * blockDim.x), d.plan.n_edges + g.n_edges, (int)(gridDim.x * blockDim.x),
+                   gridDim.x, &g);
 }
 
 // Ensemble step: one launch advances every member mesh by one of its own
@@ -1559,7 +1568,7 @@ void tiled_enqueue_step(const Dev &d, const TiledBuild &b, int step, cudaStream_
 void tiled_enqueue_cfl(const Dev &d, const TiledBuild &b, cudaStream_t s, const GateDev *gate)
 {
     if (b.plan.split) {
-        const int sides = gate ? d.m.s_num : b.plan.n_edges;
+        const int sides = b.plan.n_edges + (gate ? gate->n_edges : 0);
         int gc = (sides + 255) / 256;
         if (gc > 148 * 8) gc = 148 * 8;
         if (gc < 1) gc = 1;

@@ -40,8 +40,8 @@ def device_bytes_estimate(arrays) -> int:
     plan)."""
     e, s = arrays.e_num, arrays.s_num
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * arrays.terms + 128 * arrays.hang_cells
-    plan = 24 * e + 64 * 1024
+    scratch = 4 * (s + e + 4 * e + 3 * e + s) + 16 * ((e + 255) // 256) * arrays.terms + 136 * arrays.hang_cells
+    plan = 28 * e + 64 * 1024
     return int(arrays.nbytes() + state + scratch + plan + (1 << 20))
 
 
@@ -56,8 +56,8 @@ def device_bytes_bound(workload) -> int:
     terms = 4 + 6 * len(workload.forcing.boundaries)
     inputs = 4 * (12 * e + 8 * e + isl) + 21 * s + 16 * e + 44 * s
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 2 * e + s) + 16 * ((e + 255) // 256) * terms + 128 * hanging
-    return int(inputs + state + scratch + 24 * e + 64 * 1024 + (1 << 20))
+    scratch = 4 * (s + e + 4 * e + 3 * e + s) + 16 * ((e + 255) // 256) * terms + 136 * hanging
+    return int(inputs + state + scratch + 28 * e + 64 * 1024 + (1 << 20))
 
 
 @dataclass
