@@ -1217,6 +1217,10 @@ int plan_tiles(const HostMesh &hm, int T, std::vector<Pattern> &patterns, std::v
         }
         max_ext = std::max(max_ext, (int)ext.size());
         max_sides = std::max(max_sides, (int)sides.size());
+        // no use planning on when this tile alone is too large (the caller's
+        // shared memory holds at least these arrays)
+        if (resident ? 8LL * max_ext + 20LL * max_sides > 227 * 1024 : 32LL * max_ext + 16LL * max_sides > kMaxSharedBytes)
+            return 2;
         uint64_t hsh = pattern_hash(p);
         int found = -1;
         auto it = index.find(hsh);
@@ -1436,9 +1440,10 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         const int wave = 148 * (T == 256 ? kMinBlocks<256> : kMinBlocks<512>);
         const int n_tiles = (m.e_num + T - 1) / T;
         split = cfl_mode == 2 || (cfl_mode == 0 && (n_tiles >= 2 * wave || m.hang_cells > 0));
-        if (plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason,
-                       resident, split ? &edges : nullptr))
-            return bad(reason);
+        const int planned = plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason,
+                                       resident, split ? &edges : nullptr);
+        if (planned == 1) return bad(reason);
+        if (planned == 2) continue;
         // The budget reduction stages one term of every thread (NT doubles)
         // in the 20 * max_ext bytes of shared arrays that are dead after the
         // depth update; meshes smaller than a tile need the padding.
@@ -1456,7 +1461,10 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         smem = lean + (size_t)max_sides * 8;
         stage_sdn = smem <= (size_t)kMaxSharedBytes && resident_blocks(smem) == resident_blocks(lean);
         if (!stage_sdn) smem = lean;
-        if (resident || smem <= (size_t)kMaxSharedBytes) { tile = T; break; }
+        // A tile whose halo is several times itself is refused although it would
+        // fit: the multi-pass step is faster there (641 x 328 cells by rows, theta
+        // 0.9: 1506 us per 32 steps against 2945 with 107 KB tiles).
+        if (resident || lean + (size_t)max_ext * 4 <= (size_t)kMaxSharedBytes) { tile = T; break; }
     }
     if (!tile) return bad("tile halos exceed shared memory (cell numbering is not spatially coherent)");
     // flatten patterns
