@@ -52,6 +52,7 @@ struct Ctl {
     unsigned long long dry_key;       // the least CFL key of an all-dry state (initialize)
     uint32_t epoch, batches;          // resident form: steps and batches so far
     int32_t stalled;                  // resident form: a wait ran out
+    int32_t stepped;                  // 1 when the last slot's step ran (written by its commit only)
 };
 
 // Tile plan of the fused step (built on the host by nhf_tiled.cu).
@@ -398,6 +399,7 @@ __device__ __forceinline__ void finish_step(Ctl *c)
         row[1] = c->step_end[0]; row[2] = c->step_end[1];
         row[3] = NHF_STEP_COMPLETED;
     }
+    c->stepped = c->active;
     c->slot += 1;
 }
 

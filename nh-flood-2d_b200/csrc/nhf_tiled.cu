@@ -873,10 +873,12 @@ __global__ void __launch_bounds__(256) k_edges_tiled(const __grid_constant__ Dev
     if (blockIdx.x >= cfl_blocks) {
         const int i = (int)((blockIdx.x - cfl_blocks) * blockDim.x + threadIdx.x);
         const Ctl *c = d.ctl;
-        // the other blocks' last one prepares the next step meanwhile; where that
-        // will do nothing (or this step did), no gradients are needed, and
-        // parity does not change before the next step
-        if (!c->active) return;
+        // Nothing orders these blocks before the other blocks' last one, which
+        // prepares the next step meanwhile: they may read only what that does not
+        // write. `active` it clears and sets again (clock_choose); `stepped` and
+        // `parity` are the step launch's. A step that did nothing left the state,
+        // its gradients and the buffer that holds the last step's as they were.
+        if (!c->stepped) return;
         const int parity = c->parity;
         if (i < 2 * d.m.hang_cells && d.hang[i].cell != -1)
             (parity ? d.gradients_b : d.gradients)[i] = hang_gradient(d, cur_depth(d, parity), i >> 1, i & 1);
