@@ -153,19 +153,28 @@ __device__ __forceinline__ Faces<kTwo> faces_of(const unsigned char *table, int 
     return f;
 }
 
-// prepare_step's snapshot of the limiting side (solver_compact.py:372-382) for
-// a batch's first step, from the caller's state.
-__device__ __noinline__ void snapshot_limit(const Dev &d, float ndt, int si)
+// prepare_step's snapshot of the limiting side (solver_compact.py:372-382). Each
+// block keeps its own until the batch's end: the owner of the last one taken
+// writes it out, so the control block's words have one writer and no order
+// between blocks matters.
+struct Limit {
+    float value[5];
+    int32_t id[3];
+    int32_t mine;   // 1: the batch's last snapshot so far is this block's
+};
+
+// The snapshot of a batch's first step, from the caller's state.
+__device__ __noinline__ void snapshot_limit(const Dev &d, float ndt, int si, Limit *out)
 {
     const nhf_mesh &m = d.m;
-    Ctl *c = d.ctl;
     const int el = m.topology[3 * si + 1], eh = m.topology[3 * si + 2];
     const real h = flow_depth_of(m, m.depth, si);
-    c->limit_value[0] = ndt;
-    c->limit_value[1] = m.depth[el]; c->limit_value[2] = m.depth[eh];
-    c->limit_value[3] = h;
-    c->limit_value[4] = m.q[si] / rmax(h, RC(1e-30));
-    c->limit_ids[0] = si; c->limit_ids[1] = el; c->limit_ids[2] = eh;
+    out->value[0] = ndt;
+    out->value[1] = m.depth[el]; out->value[2] = m.depth[eh];
+    out->value[3] = h;
+    out->value[4] = m.q[si] / rmax(h, RC(1e-30));
+    out->id[0] = si; out->id[1] = el; out->id[2] = eh;
+    out->mine = 1;
 }
 
 template <bool kThetaOne, bool kTwo, int NT, int T>
@@ -185,6 +194,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
     __shared__ uint32_t sh_row[NHF_TRACE_COLS], sh_end[NHF_MAX_BATCH][2];
     __shared__ float sh_ndt;
     __shared__ int sh_arg, sh_slot, sh_hang, sh_last;
+    __shared__ Limit sh_limit;
 
     const nhf_mesh &m = d.m;
     Ctl *c = d.ctl;
@@ -233,7 +243,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
         ck.now[0] = c->now[0]; ck.now[1] = c->now[1];
         ck.next[0] = r.words[0]; ck.next[1] = r.words[1];
         ck.origin[0] = r.words[2]; ck.origin[1] = r.words[3];
-        sh_ndt = c->ndt; sh_arg = c->cfl_arg; sh_slot = 0; sh_hang = 0;
+        sh_ndt = c->ndt; sh_arg = c->cfl_arg; sh_slot = 0; sh_hang = 0; sh_limit.mine = 0;
         sh_cnt[0] = sh_cnt[1] = sh_cnt[2] = 0u; sh_minbits = __float_as_uint(1.0f);
         sh_s[0] = 0.0f;  // donor factor of the exterior sentinel
         sh_q[n_sides] = sh_len[n_sides] = 0.0f;
@@ -337,7 +347,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
     };
     if (tid == 0) {
         choose(0, blockIdx.x == 0 ? c->trace : sh_row);
-        if (ck.active && sh_ndt < limit0 && blockIdx.x == 0) snapshot_limit(d, sh_ndt, sh_arg);
+        if (ck.active && sh_ndt < limit0 && blockIdx.x == 0) snapshot_limit(d, sh_ndt, sh_arg, &sh_limit);
     }
     if constexpr (kTwo) {
         for (int k = tid; k < 2 * n_hang; k += NT) {
@@ -744,15 +754,18 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
             if (slot_now + 1 < batch && ck.active && ndt < limit0) {
                 // the limiting side's snapshot (372-382), by its owner
                 limit0 = ndt;
-                if (lane == 0 && least == best && least != ~kPhase) {
-                    const uint32_t lh = sh_lohi[best_side];
-                    const int a = (int)(lh & kSlot), b = (int)((lh >> 16) & kSlot);
-                    const float h = cfl_face_depth(sh_z[a], sh_h[a], sh_z[b], sh_h[b]);
-                    c->limit_value[0] = ndt;
-                    c->limit_value[1] = sh_h[a]; c->limit_value[2] = sh_h[b];
-                    c->limit_value[3] = h;
-                    c->limit_value[4] = sh_q[best_side] / rmax(h, RC(1e-30));
-                    c->limit_ids[0] = arg; c->limit_ids[1] = cbase + ext[a]; c->limit_ids[2] = cbase + ext[b];
+                if (lane == 0) {
+                    sh_limit.mine = least == best && least != ~kPhase;
+                    if (sh_limit.mine) {
+                        const uint32_t lh = sh_lohi[best_side];
+                        const int a = (int)(lh & kSlot), b = (int)((lh >> 16) & kSlot);
+                        const float h = cfl_face_depth(sh_z[a], sh_h[a], sh_z[b], sh_h[b]);
+                        sh_limit.value[0] = ndt;
+                        sh_limit.value[1] = sh_h[a]; sh_limit.value[2] = sh_h[b];
+                        sh_limit.value[3] = h;
+                        sh_limit.value[4] = sh_q[best_side] / rmax(h, RC(1e-30));
+                        sh_limit.id[0] = arg; sh_limit.id[1] = cbase + ext[a]; sh_limit.id[2] = cbase + ext[b];
+                    }
                 }
             }
         } else {
@@ -830,6 +843,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
         const size_t g = (size_t)blk * terms_n + i % terms_n;
         if (blk < d.blocks) { d.acc_sum[g] = sh_acc[2 * i]; d.acc_comp[g] = sh_acc[2 * i + 1]; }
     }
+    if (tid < 5 && sh_limit.mine) c->limit_value[tid] = sh_limit.value[tid];
+    if (tid < 3 && sh_limit.mine) c->limit_ids[tid] = sh_limit.id[tid];
     if (epoch != epoch0)
         for (int j = tid; j < n_owned; j += NT) m.q[sh_gid[j]] = sh_q[j];
 #pragma unroll
