@@ -29,6 +29,7 @@ constexpr int kBlock = 256;                 // budget block = reference ei // 25
 constexpr real kDh = RC(-999.0);            // dh_t without gates (solver_compact.py:405)
 constexpr uint32_t kSnapTicks = 1099512u;   // ceil(1e-6 * 2**40) (clock.py:11)
 constexpr unsigned long long kCflEmpty = 0xFFFFFFFFFFFFFFFFULL;
+constexpr uint32_t kCflNan = 0x80000000u;   // in Ctl::done_blocks: the step's dry CFL key may not hold (note_cfl_nan)
 
 // Device control block: the reference's scalar fields (clock words, dt,
 // limiter counters, CFL result, limiting-edge snapshot) and the batch trace.
@@ -283,6 +284,56 @@ __device__ __forceinline__ float fastest_speed(bool wet, float qx, float qy, flo
     const float s2 = u * u + v * v;
     const float speed = s2 == 0.0f ? 0.0f : sqrtf(s2);
     return speed > fastest ? speed : fastest;
+}
+
+// The dry key stands for the sides at the face depth's floor without discharge as
+// long as its own side's CFL value is a number. Where it may not be, a thread
+// notes so beside the count of finished blocks before its block adds itself, so
+// that the last block knows without a read of its own on the step's serial end
+// (a word of its own, or a test of the result, cost 0.9 us a step there).
+__device__ __forceinline__ void note_cfl_nan(Ctl *c) { atomicOr(&c->done_blocks, kCflNan); }
+
+// 0, or for the last of `blocks` blocks 1, and 2 where the dry key may not hold.
+__device__ __forceinline__ int last_of(uint32_t ticket, uint32_t blocks)
+{
+    return (ticket & ~kCflNan) == blocks - 1 ? 1 + (int)(ticket >> 31) : 0;
+}
+
+// A step's CFL result: the least of the blocks' keys and the dry key, or `exact`
+// of all sides' keys (rescan_cfl).
+__device__ __forceinline__ void set_cfl(Ctl *c, bool exact)
+{
+    const unsigned long long all = atomicExch(&c->cfl_packed, kCflEmpty);
+    const unsigned long long packed = c->dry_key < all && !exact ? c->dry_key : all;
+    if (packed == kCflEmpty) {
+        c->ndt = __uint_as_float(0x7f800000u);
+        c->cfl_arg = 0;
+    } else {
+        c->ndt = __uint_as_float((uint32_t)(packed >> 32));
+        c->cfl_arg = (int32_t)(packed & 0xffffffffu);
+    }
+}
+
+// The least key of every interior side of a state (depths of cells, discharges of
+// sides) into the control block, by all threads of the last block; a value that is
+// not a number is above every other.
+template <class State>
+__device__ __noinline__ void rescan_cfl(const Dev &d, const State state)
+{
+    const nhf_mesh &m = d.m;
+    unsigned long long best = kCflEmpty;
+    __threadfence();
+    for (int si = 1 + (int)threadIdx.x; si < m.s_num; si += (int)blockDim.x) {
+        const int el = m.topology[3 * si + 1], eh = m.topology[3 * si + 2];
+        if (el == 0 || eh == 0) continue;
+        const real h = cfl_face_depth(m.bed[el], state.depth(el), m.bed[eh], state.depth(eh));
+        const real value = cfl_value(d.afa, d.g, m.length[si], state.q(si), h);
+        const unsigned long long key = ((unsigned long long)__float_as_uint(value) << 32) | (unsigned)si;
+        best = key < best ? key : best;
+    }
+    best = warp_min_key(best);
+    if ((threadIdx.x & 31) == 0 && best != kCflEmpty) atomicMin(&d.ctl->cfl_packed, best);
+    __syncthreads();
 }
 #endif
 

@@ -235,6 +235,18 @@ __device__ __forceinline__ void lattice_cfl(const Dev &d, real len, real q, real
     }
 }
 
+// The state of buffer `p`, for rescan_cfl.
+struct LatticeState {
+    const LatticePlan *P;
+    int p;
+    __device__ __forceinline__ real depth(int cell) const { return __ldcg(P->h[p] + P->glat[cell]); }
+    __device__ __forceinline__ real q(int side) const
+    {
+        const int at = P->gside[side];
+        return __ldcg(((at & 1) ? P->qh[p] : P->qv[p]) + (at >> 1));
+    }
+};
+
 // prepare_step (solver_compact.py:364-382) with the state in lattice order.
 __device__ __noinline__ void lattice_prepare(const Dev &d, Ctl *c)
 {
@@ -472,13 +484,17 @@ __global__ void __launch_bounds__(256, 6) k_lattice_close(const __grid_constant_
 {
     __shared__ unsigned long long sh_min[8];
     __shared__ uint32_t sh_cnt[8][4];
-    __shared__ bool last;
+    __shared__ int last;
     const LatticePlan &P = d.lat;
     const nhf_mesh &m = d.m;
     Ctl *c = d.ctl;
     const int tid = threadIdx.x;
     const size_t e = (size_t)m.e_num;
     const int T = d.terms;
+    // the last block's first thread looks at the dry key's own side (a value that
+    // is not a number has no finite discharge)
+    const int dry_side = blockIdx.x == gridDim.x - 1 && tid == 0 ? (int)(uint32_t)c->dry_key : -1;
+    const int dry_at = dry_side > 0 ? P.gside[dry_side] : 0;
     // a warp looks at an even share of the budget blocks' marks, 32 at most at a
     // time, and takes the marked ones: lane l holds the tree's slots l, l + 32, .. l + 224, so the strides 128, 64 and
     // 32 are its own sums and a shuffle tree does 16 .. 1
@@ -522,6 +538,7 @@ __global__ void __launch_bounds__(256, 6) k_lattice_close(const __grid_constant_
             best = P.part_cfl[w] < best ? P.part_cfl[w] : best;
         }
         const int p = c->parity ^ 1;  // the state the march just wrote
+        const real dry_q = dry_side > 0 ? ((dry_at & 1) ? P.qh[p] : P.qv[p])[dry_at >> 1] : RC(0);
         const real *h = P.h[p], *qh = P.qh[p];
         const size_t lx = (size_t)P.lx;
         // counts below 2^31: the planner keeps the lattice under 2^30 points
@@ -545,6 +562,7 @@ __global__ void __launch_bounds__(256, 6) k_lattice_close(const __grid_constant_
                                 best);
             }
         }
+        if (!(fabs(dry_q) < __uint_as_float(0x7f800000u))) note_cfl_nan(c);
     }
     best = warp_min_u64(best);
     lim = __reduce_add_sync(0xffffffffu, lim);
@@ -573,22 +591,16 @@ __global__ void __launch_bounds__(256, 6) k_lattice_close(const __grid_constant_
         if (wt) atomicAdd(&c->wet, wt);
         __threadfence();
         const unsigned ticket = atomicAdd(&c->done_blocks, 1u);
-        last = ticket == gridDim.x - 1;
+        last = last_of(ticket, gridDim.x);
     }
     __syncthreads();
-    if (!last || tid != 0) return;
+    if (!last) return;
+    if (last == 2) rescan_cfl(d, LatticeState{&P, c->parity ^ 1});
+    if (tid != 0) return;
     __threadfence();
-    unsigned long long packed = atomicExch(&c->cfl_packed, kCflEmpty);
-    packed = c->dry_key < packed ? c->dry_key : packed;
     c->done_blocks = 0;
     if (active) {
-        if (packed == kCflEmpty) {
-            c->ndt = __uint_as_float(0x7f800000u);
-            c->cfl_arg = 0;
-        } else {
-            c->ndt = __uint_as_float((uint32_t)(packed >> 32));
-            c->cfl_arg = (int32_t)(packed & 0xffffffffu);
-        }
+        set_cfl(c, last == 2);
         c->parity ^= 1;
     }
     finish_step(c);

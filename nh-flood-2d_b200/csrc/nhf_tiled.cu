@@ -199,28 +199,24 @@ __device__ __forceinline__ float term_value(int t, int B, float removed, float f
 // face depth's floor with no discharge is left to the dry key (the least key
 // of an all-dry state, folded in with the result): no side's value is above
 // its dry one, so where the minimum is that small the dry key's sides attain it.
+// `note`: a value that is not a number is noted.
 __device__ __forceinline__ void fold_cfl(const Dev &d, float len, float q, float h, unsigned gid,
-                                         unsigned long long &best)
+                                         unsigned long long &best, bool note = false)
 {
     if (h == 0.01f && q == 0.0f) return;
     if (cfl_above(d.afa * len, d.g, q, h, __uint_as_float((uint32_t)(best >> 32)))) return;
-    const unsigned long long key = ((unsigned long long)__float_as_uint(cfl_value(d.afa, d.g, len, q, h)) << 32) | gid;
+    const uint32_t bits = __float_as_uint(cfl_value(d.afa, d.g, len, q, h));
+    if (note && bits > 0x7f800000u) note_cfl_nan(d.ctl);
+    const unsigned long long key = ((unsigned long long)bits << 32) | gid;
     best = key < best ? key : best;
 }
 
-// The step's CFL result: the least of the blocks' keys and the dry key.
-__device__ __forceinline__ void set_cfl(Ctl *c)
-{
-    const unsigned long long all = atomicExch(&c->cfl_packed, kCflEmpty);
-    const unsigned long long packed = c->dry_key < all ? c->dry_key : all;
-    if (packed == kCflEmpty) {
-        c->ndt = __uint_as_float(0x7f800000u);
-        c->cfl_arg = 0;
-    } else {
-        c->ndt = __uint_as_float((uint32_t)(packed >> 32));
-        c->cfl_arg = (int32_t)(packed & 0xffffffffu);
-    }
-}
+// The state that a tiled step wrote, for rescan_cfl.
+struct TiledState {
+    const float *h, *qs;
+    __device__ __forceinline__ float depth(int cell) const { return __ldcg(h + cell); }
+    __device__ __forceinline__ float q(int side) const { return __ldcg(qs + side); }
+};
 
 // One fused step of tile t of the mesh described by d (n_tiles tiles).
 // kHang: 0 no hanging edges, 1 hanging edges, 2 decided by d at run time.
@@ -735,7 +731,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             float zl = sh_z[a], zh = sh_z[b];
             float head = maxf(zl + sh_s[a], zh + sh_s[b]);
             float h = rmaxc(head - rmaxc(maxf(zl, zh), kDh), 0.01f);
-            fold_cfl(d, sh_len[j], qv, h, (unsigned)gid, best);
+            fold_cfl(d, sh_len[j], qv, h, (unsigned)gid, best, !split);
         }
     }
     if (last_cell) {
@@ -758,16 +754,18 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
         if (sh_cnt[2]) atomicAdd(&c->wet, sh_cnt[2]);
         __threadfence();
         unsigned ticket = atomicAdd(&c->done_blocks, 1u);
-        sh_last = ticket == n_tiles - 1;
+        sh_last = last_of(ticket, n_tiles);
     }
     __syncthreads();
-    if (!sh_last || tid != 0) return;
+    if (!sh_last) return;
     // Last block: (fused-CFL form: the CFL result,) trace row, clock commit,
     // the new state becomes current (and the next step is prepared).
+    if (sh_last == 2) rescan_cfl(d, TiledState{depth_out, q_out});
+    if (tid != 0) return;
     __threadfence();
     c->done_blocks = 0;
     if (!split) {
-        set_cfl(c);
+        set_cfl(c, sh_last == 2);
     }
     finish_step(c);
     c->grad_parity = gradients == d.gradients ? 0 : 1;
@@ -775,23 +773,25 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     if (!split && c->slot < d.batch_size) prepare_step(d, c, depth_out, q_out);
 }
 
-// CFL pass (solver_compact.py:617-641) over sides [first, end) with stride (or,
-// kEdges, over the plan's sides between tiles), on the current (just updated)
-// state; each block adds its minimum packed key (cfl bits, side id) and the
+// CFL pass (solver_compact.py:617-641), block `block` of `blocks`, over sides
+// [first, end) with stride (or, kEdges, over the plan's sides between tiles), on
+// the current (just updated) state; each block adds its minimum packed key (cfl bits, side id) and the
 // last of `blocks` blocks sets ndt / cfl_arg (the lowest side id attains the
 // minimum) and prepares the next step (solver_compact.py:364-382).
 template <bool kEdges = false>
-__device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int stride, unsigned blocks,
+__device__ __forceinline__ void cfl_pass(const Dev &d, unsigned block, unsigned blocks, int first, int end, int stride,
                                          const GateDev *gd = nullptr)
 {
     __shared__ unsigned long long sh[32];
-    __shared__ bool last;
-    __shared__ int prepared;
+    __shared__ int last, prepared;
     const nhf_mesh &m = d.m;
     Ctl *c = d.ctl;
     const int active = c->active;
     const float *depth = cur_depth(d, c->parity);
     const float *q = cur_q(d, c->parity);
+    // the last block's first thread looks at the dry key's own side (a value that
+    // is not a number has no finite discharge)
+    const int dry_side = block == blocks - 1 && threadIdx.x == 0 ? (int)(uint32_t)c->dry_key : -1;
     // sides between tiles start from the minimum of those inside
     unsigned long long best = kEdges ? __ldcg(&c->cfl_packed) : kCflEmpty;
     if (active) {
@@ -811,6 +811,7 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
             }
         }
     }
+    if (dry_side > 0 && active && !(fabsf(q[dry_side]) < __uint_as_float(0x7f800000u))) note_cfl_nan(c);
     best = warp_min_u64(best);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) sh[warp] = best;
@@ -822,15 +823,16 @@ __device__ __forceinline__ void cfl_pass(const Dev &d, int first, int end, int s
             if (best != kCflEmpty) atomicMin(&c->cfl_packed, best);
             __threadfence();
             const unsigned ticket = atomicAdd(&c->done_blocks, 1u);
-            last = ticket == blocks - 1;
+            last = last_of(ticket, blocks);
         }
     }
     __syncthreads();
     if (!last) return;
+    if (last == 2) rescan_cfl(d, TiledState{depth, q});
     if (threadIdx.x == 0) {
         __threadfence();
         c->done_blocks = 0;
-        if (active) set_cfl(c);
+        if (active) set_cfl(c, last == 2);
         prepared = c->slot < d.batch_size;
         if (prepared) prepare_step(d, c, depth, q);
     }
@@ -884,15 +886,16 @@ __global__ void __launch_bounds__(256) k_edges_tiled(const __grid_constant__ Dev
             (parity ? d.gradients_b : d.gradients)[i] = hang_gradient(d, cur_depth(d, parity), i >> 1, i & 1);
         return;
     }
-    cfl_pass<true>(d, (int)(blockIdx.x * blockDim.x), d.plan.n_edges, (int)(cfl_blocks * blockDim.x), cfl_blocks);
+    cfl_pass<true>(d, blockIdx.x, cfl_blocks, (int)(blockIdx.x * blockDim.x), d.plan.n_edges,
+                   (int)(cfl_blocks * blockDim.x));
 }
 
 // The same CFL pass of a gate run (split plan), after the beds have moved: the
 // sides between tiles and those of gate cells; also the next step's check_gates.
 __global__ void __launch_bounds__(256) k_cfl_tiled_gate(const __grid_constant__ Dev d, const __grid_constant__ GateDev g)
 {
-    cfl_pass<true>(d, (int)(blockIdx.x * blockDim.x), d.plan.n_edges + g.n_edges, (int)(gridDim.x * blockDim.x),
-                   gridDim.x, &g);
+    cfl_pass<true>(d, blockIdx.x, gridDim.x, (int)(blockIdx.x * blockDim.x), d.plan.n_edges + g.n_edges,
+                   (int)(gridDim.x * blockDim.x), &g);
 }
 
 // Ensemble step: one launch advances every member mesh by one of its own
@@ -1358,7 +1361,7 @@ __global__ void __launch_bounds__(256) k_ens_cfl(const Dev *devs, const int2 *it
     const int n = d.m.e_num > d.m.s_num ? d.m.e_num : d.m.s_num;
     const unsigned chunks = (unsigned)((n + kEnsChunk - 1) / kEnsChunk);
     const int first = max(1, w.y * kEnsChunk), end = min(d.m.s_num, (w.y + 1) * kEnsChunk);
-    cfl_pass(d, first, end, (int)blockDim.x, chunks);
+    cfl_pass(d, (unsigned)w.y, chunks, first, end, (int)blockDim.x);
 }
 
 // Batch end, part 1: the current state back into the caller's buffers.
@@ -1579,9 +1582,8 @@ void tiled_enqueue_cfl(const Dev &d, const TiledBuild &b, cudaStream_t s, const 
 {
     if (b.plan.split) {
         const int sides = b.plan.n_edges + (gate ? gate->n_edges : 0);
-        int gc = (sides + 255) / 256;
+        int gc = (sides + 255) / 256 + 1;   // one more, which looks at the dry key's side
         if (gc > 148 * 8) gc = 148 * 8;
-        if (gc < 1) gc = 1;
         if (gate) k_cfl_tiled_gate<<<gc, 256, 0, s>>>(d, *gate);
         else k_edges_tiled<<<gc + (2 * d.m.hang_cells + 255) / 256, 256, 0, s>>>(d, (unsigned)gc);
     }
