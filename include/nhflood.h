@@ -113,8 +113,8 @@ typedef struct nhf_params {
     int32_t path;       /* 0: the resident form (the whole batch in one
                            cooperative launch) when one tile per SM covers
                            the mesh, else the lattice form on a uniform grid
-                           it covers of at least 2^18 cells, else the fused
-                           tiled step when the mesh allows it, else
+                           it covers of at least 2^18 cells (2^20 with
+                           cfl_mode 2), else the fused tiled step when the mesh allows it, else
                            multi-pass; 4: the same without the resident form
                            (members of an ensemble, which run beside others); 1: always the multi-pass step;
                            2: the lattice form when the mesh allows it, else

@@ -1046,8 +1046,11 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     // Lattice form when the mesh is a uniform grid it covers (params->path 2, or
     // a grid of at least 2^18 cells that does not run resident: 600 x 600 cells
     // 1357 us per 32 steps against 1603 on tiles, 1003 x 741 2047 against 2806
-    // (numbered by rows 2054 against 4580), 421 x 307 1037 against 983).
-    if (!h->resident && (params->path == 2 || (any_form && mesh->e_num - 1 >= (1 << 18)))) {
+    // (numbered by rows 2054 against 4580), 421 x 307 1037 against 983). A caller
+    // that places the CFL in a pass of its own keeps the tiles up to 2^20 cells,
+    // where a gate controller can be attached to them.
+    const int lattice_from = params->cfl_mode == 2 ? 1 << 20 : 1 << 18;
+    if (!h->resident && (params->path == 2 || (any_form && mesh->e_num - 1 >= lattice_from))) {
         Dev probe{};
         probe.m = *mesh;
         probe.terms = 4 + 6 * mesh->b_num;

@@ -1,0 +1,49 @@
+"""Handles that take a gate controller after they are made: every choice of step
+that leads to 256-cell tiles with a separate CFL pass, or to the multi-pass step,
+runs as the gated engine does, bit for bit."""
+import numpy as np
+import pytest
+
+from test_gpu_resident import FIELDS
+
+pytestmark = pytest.mark.gpu
+
+
+def attached_later(path, cfl):
+    """An engine made without the controller, which is attached then."""
+    def factory(arrays, params):
+        from nhflood.native import CudaEngine
+        tables, arrays.gate = arrays.gate, None
+        params.path, params.cfl = path, cfl
+        try:
+            engine = CudaEngine(arrays, params)
+        finally:
+            arrays.gate = tables
+        engine.gate = tables
+        engine._attach_gate(tables)
+        return engine
+    return factory
+
+
+@pytest.mark.parametrize('n, path, cfl', [
+    (512, 'auto', 'pass'),      # 262,144 cells: the lattice form's size from 2^18 on
+    (549, 'auto', 'pass'),      # 301,401: the largest with 256-cell tiles
+    (128, 'auto', 'pass'),
+    (96, 'multipass', 'auto'),
+])
+def test_gate_attached_later(cuda_available, n, path, cfl):
+    from nhflood.native import CudaEngine
+    from nhflood.plain import PlainRun
+    from nhflood.workloads import gated_polder
+    w = gated_polder(n=n, duration=600)
+    runs = [PlainRun(w, f) for f in (attached_later(path, cfl), lambda a, p: CudaEngine(a, p))]
+    for _ in range(2):
+        a, b = (r.engine.run_batch(*r.begin()) for r in runs)
+        np.testing.assert_array_equal(a, b)
+        for r in runs:
+            r.finish(a)
+    for field in FIELDS + ('bed',):
+        np.testing.assert_array_equal(*(r.engine.get(field).view(np.uint32) for r in runs), field)
+    np.testing.assert_array_equal(*(r.engine.gate_flush() for r in runs))
+    for r in runs:
+        r.close()
