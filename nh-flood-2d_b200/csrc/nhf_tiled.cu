@@ -1439,10 +1439,12 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     for (int T : sizes) {
         // The separate CFL pass pays one launch per step for less halo work
         // (no ring 3, no ring-1 depth recompute): worth it from two waves of
-        // resident blocks on, and wherever there are hanging edges, whose
+        // five 256-cell tiles or two larger ones per SM on (32 steps on 256-cell
+        // tiles, in the step and in a pass: 600 x 600 cells 1333 and 1340 us, 640 x
+        // 640 1457 and 1418), and wherever there are hanging edges, whose
         // gradients take a launch in either form (32 steps of 0.19 M cells 1263
         // to 1016 us, of six members of 1.2 M cells together 5067 to 4235).
-        const int wave = 148 * (T == 256 ? kMinBlocks<256> : kMinBlocks<512>);
+        const int wave = 148 * (T == 256 ? 5 : 2);
         const int n_tiles = (m.e_num + T - 1) / T;
         split = cfl_mode == 2 || (cfl_mode == 0 && (n_tiles >= 2 * wave || m.hang_cells > 0));
         const int planned = plan_tiles(hm, T, patterns, tp, tc, ts, max_ext, max_sides, max_faces, split ? 2 : 3, reason,

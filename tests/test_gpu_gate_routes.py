@@ -30,6 +30,7 @@ def attached_later(path, cfl):
     (549, 'auto', 'pass'),      # 301,401: the largest with 256-cell tiles
     (128, 'auto', 'pass'),
     (96, 'multipass', 'auto'),
+    (616, 'tile256', 'auto'),   # 1,483 tiles: the pass by size
 ])
 def test_gate_attached_later(cuda_available, n, path, cfl):
     from nhflood.native import CudaEngine
