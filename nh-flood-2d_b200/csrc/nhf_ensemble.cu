@@ -179,7 +179,8 @@ int nhf_ensemble_create(nhf_handle *const *members, int32_t n, int32_t grid_bloc
     if (grid_blocks == -2) return create_member_graphs(members, n, stream, out);
     for (int i = 0; i < n; ++i) {
         if (!members[i]) return efail(nullptr, NHF_EINVAL, "member %d is null", i);
-        step_plan(members[i]);
+        const int rc = step_plan(members[i]);
+        if (rc) return efail(nullptr, rc, "member %d: %s", i, members[i]->err.c_str());
     }
     const int tile = h0->tb.plan.tile;
     for (int i = 0; i < n; ++i) {

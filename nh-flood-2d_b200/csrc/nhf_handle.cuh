@@ -34,6 +34,7 @@ struct nhf_handle {
     bool resident = false;      // batches of this handle run resident; its step plan (tb) is made when a graph needs it
     nhf::GateDev gate{};
     bool gate_on = false;
+    void *step_mem = nullptr;   // second state buffers of a lattice handle in a one-launch ensemble
     void *gate_mem = nullptr;   // gate budget partials
     void *gate_edges = nullptr; // sides of gate cells inside tiles (fused step)
     double *h_gacc = nullptr;   // pinned staging of the gate partials
@@ -44,7 +45,9 @@ struct nhf_handle {
 
 namespace nhf {
 // The tile plan of the step-by-step form, for a handle whose own batches run
-// resident and that joins an ensemble. NHF_OK, or an error code.
+// resident and that joins an ensemble, or whose size alone chose the lattice form
+// (fewer than 2^20 cells) and that joins a one-launch ensemble. NHF_OK, or an
+// error code.
 int step_plan(nhf_handle *h);
 // The ensemble's member-graph schedule (nhf_step.cu): build a member's batch
 // graph, and launch it on the member's stream after `start`, recording `done`.

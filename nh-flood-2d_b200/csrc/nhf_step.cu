@@ -67,6 +67,15 @@ __global__ void k_initialize(Dev d)
     }
 }
 
+#ifndef NHF_REAL_DOUBLE
+// The tiled step's centre distances and Manning n, for a handle that is initialized.
+__global__ void k_sdn(Dev d)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < d.m.s_num) d.sdn[i] = i ? make_float2(d.sdc[i], d.m.side_n[i]) : make_float2(0.0f, 0.0f);
+}
+#endif
+
 // clock.begin on the device (clock.py:75-92): the target and origin words are
 // kernel arguments, updated in the instantiated graph before each replay. The
 // tiled form also prepares slot 0 here (each fused step prepares the next).
@@ -871,7 +880,7 @@ void enqueue_step(nhf_handle *h)
 int build_graph(nhf_handle *h)
 {
     cudaGraph_t g = nullptr;
-    int rc = step_plan(h);
+    int rc = h->resident ? step_plan(h) : NHF_OK;
     if (rc) return rc;
     CK(h, cudaStreamBeginCapture(h->s, cudaStreamCaptureModeThreadLocal));
     k_begin<<<1, 256, 0, h->s>>>(h->dev, 0u, 0u, 0u, 0u, (h->tiled || h->lattice) ? 1 : 0);
@@ -939,10 +948,35 @@ namespace nhf {
 int step_plan(nhf_handle *h)
 {
 #ifndef NHF_REAL_DOUBLE
-    if (!h->resident || h->tb.device_memory) return NHF_OK;
+    const bool chosen_lattice = h->lattice && h->p.path != 2 && h->m.e_num - 1 < (1 << 20);
+    if (!(h->resident || chosen_lattice) || h->tb.device_memory) return NHF_OK;
     char why[256] = {0};
     h->tiled = tiled_build(h->m, h->s, &h->tb, why, sizeof(why), 0, h->p.cfl_mode) == 0;
-    if (h->tiled) h->dev.plan = h->tb.plan;   // otherwise the graph takes the multi-pass step
+    if (!h->tiled) return NHF_OK;   // the graph takes the multi-pass step, or the lattice
+    if (h->lattice) {   // the state's second buffers, which a lattice handle has none of
+        const size_t e = sizeof(real) * (size_t)h->m.e_num, sn = (size_t)h->m.s_num;
+        auto up = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+        char *mem = nullptr;
+        if (cudaMalloc((void **)&mem, 3 * up(e) + up(sizeof(real) * sn) + up(sizeof(float2) * sn)) != cudaSuccess) {
+            cudaGetLastError();
+            cudaFree(h->tb.device_memory);
+            h->tb.device_memory = nullptr;
+            h->tiled = false;
+            return NHF_OK;
+        }
+        h->step_mem = mem;
+        Dev &d = h->dev;
+        d.depth_b = (real *)mem;
+        d.rain_time_b = (real *)(mem + up(e));
+        d.rain_rate = (real *)(mem + 2 * up(e));
+        d.q_b = (real *)(mem + 3 * up(e));
+        d.sdn = (float2 *)(mem + 3 * up(e) + up(sizeof(real) * sn));
+        CK(h, cudaMemsetAsync(mem, 0, 3 * up(e) + up(sizeof(real) * sn), h->s));
+        k_sdn<<<grid_for(h->m.s_num, 256), 256, 0, h->s>>>(d);
+        CK(h, cudaGetLastError());
+        CK(h, cudaStreamSynchronize(h->s));
+    }
+    h->dev.plan = h->tb.plan;
 #endif
     return NHF_OK;
 }
@@ -1186,6 +1220,7 @@ int nhf_destroy(nhf_handle *h)
     if (h->graph_def) cudaGraphDestroy(h->graph_def);
     if (h->tb.device_memory) cudaFree(h->tb.device_memory);
     if (h->lb.device_memory) cudaFree(h->lb.device_memory);
+    if (h->step_mem) cudaFree(h->step_mem);
     if (h->rb.tables) cudaFree(h->rb.tables);
     if (h->rb.memory) cudaFree(h->rb.memory);
     if (h->scratch) cudaFree(h->scratch);
