@@ -1417,7 +1417,9 @@ int nhf_gate_attach(nhf_handle *h, const nhf_gate *gate)
     if (h->lattice)
         return fail(h, NHF_EINVAL, "gate control runs on the multi-pass step or the fused tiled step, not the "
                                    "lattice form (nhf_params.path = 1, or 256 with cfl_mode 2)");
-    if (h->tiled && !(h->tb.plan.tile == 256 && h->tb.plan.split))
+    // (a resident handle's batches have no gate passes, whatever step plan an
+    // ensemble has given it)
+    if (h->resident || (h->tiled && !(h->tb.plan.tile == 256 && h->tb.plan.split)))
         return fail(h, NHF_EINVAL, "gate control runs on the multi-pass step or on the fused step with 256-cell "
                                    "tiles and the separate CFL pass (nhf_params.path = 1, or 256 with cfl_mode 2)");
     if (h->gate_on) return fail(h, NHF_ESTATE, "a gate controller is already attached");

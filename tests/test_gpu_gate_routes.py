@@ -48,3 +48,26 @@ def test_gate_attached_later(cuda_available, n, path, cfl):
     np.testing.assert_array_equal(*(r.engine.gate_flush() for r in runs))
     for r in runs:
         r.close()
+
+
+def test_resident_handle_of_an_ensemble_is_refused(cuda_available):
+    """A resident handle takes no controller, before and after an ensemble has
+    given it a plan of 256-cell tiles with a separate pass."""
+    from test_gpu_resident import quadtree
+    from nhflood.gate import GateTables
+    from nhflood.native import CudaEngine, CudaEnsemble
+    from nhflood.plain import PlainRun
+    w = quadtree(1200)
+    e = w.mesh.e_num
+    none = np.zeros(0, np.int32)
+    tables = GateTables(1, np.full(e, -1, np.int32), np.zeros(e, np.int32), np.zeros(e, np.float32), none,
+                        np.ones(1, np.int32), none, 0, 1.0, 1.0, 0.0)
+    run = PlainRun(w, lambda a, p: CudaEngine(a, p))
+    assert 'resident=' in run.engine.path
+    with pytest.raises(RuntimeError, match='gate control runs'):
+        run.engine._attach_gate(tables)
+    ens = CudaEnsemble([run.engine], -2)
+    with pytest.raises(RuntimeError, match='gate control runs'):
+        run.engine._attach_gate(tables)
+    ens.close()
+    run.close()
