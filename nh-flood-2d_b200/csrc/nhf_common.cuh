@@ -114,7 +114,7 @@ struct LatticePlan {
     float *terms;                   // [terms][e_num] budget terms of a step by global id, else zero
     uint32_t *touched;              // [blocks] terms but 0 some cell of a 256-cell budget block holds
     uint8_t *touched_rain;          // [blocks] 1 where some cell holds term 0 (infiltration)
-    int32_t *odd;                   // 1 during a batch that starts with extrema below zero
+    int32_t *odd;                   // 1 during a batch whose dry cells may change (k_lattice_gather)
     uint8_t *plain;                 // [chunks*strips] 1: the warp's cells are live and off the boundaries
     uint32_t *part;                 // [4][strips*chunks] per-warp limited cells, limited faces, wet cells, min scale bits
     unsigned long long *part_cfl;   // [strips*chunks] per-warp CFL key

@@ -293,7 +293,7 @@ __device__ __forceinline__ void lattice_rows(const Dev &d, const int strip, cons
     const Ctl *c = d.ctl;
     const real dt = c->dt;
     const bool raining = c->raining != 0;
-    const bool horton = raining && P.horton, keep_idle = *P.odd == 0;
+    const bool horton = raining && P.horton, keep_idle = *P.odd == 0 && d.min_h > RC(0);
     const real one_rate = raining && !P.rain_cells ? d.rain_rates[0] : RC(0);
     const real *h_in = P.h[kParity], *qv_in = P.qv[kParity], *qh_in = P.qh[kParity];
     real *h_out = P.h[1 - kParity], *qv_out = P.qv[1 - kParity], *qh_out = P.qh[1 - kParity];
@@ -391,7 +391,7 @@ __device__ __forceinline__ void lattice_rows(const Dev &d, const int strip, cons
         // use; none for a row whose cells are dry and stay dry (no rain, no
         // discharge on any side), which saves their 20 bytes a cell
         k0 = LatticeCell{0, b1, RC(0), RC(0), RC(0), RC(0), RC(0), RC(0), RC(0)};
-        const bool moves = qw1 != RC(0) || qe1 != RC(0) || qs1 != RC(0) || qs2 != RC(0) || h1 != RC(0) || r1 > RC(0);
+        const bool moves = qw1 != RC(0) || qe1 != RC(0) || qs1 != RC(0) || qs2 != RC(0) || h1 != RC(0) || r1 != RC(0);
         busy = __any_sync(kAll, own && moves) || !keep_idle;
         if (own && (kPlain ? busy : l1) && y + 1 >= y0 && y + 1 < y1) {
             k0.infil = get(P.infil, o1);
@@ -645,8 +645,9 @@ __global__ void k_lattice_gather(const __grid_constant__ Dev d)
             P.infil[L] = m.infiltration[g];
             P.max_depth[L] = m.max_depth[g];
             P.max_speed[L] = m.max_speed[g];
-            // extrema below zero would rise to a dry cell's zero: no idle rows then
-            if (m.max_depth[g] < RC(0) || m.max_speed[g] < RC(0)) *P.odd = 1;
+            // extrema below zero would rise to a dry cell's zero, and infiltration
+            // below zero would wet it: no idle rows then
+            if (m.max_depth[g] < RC(0) || m.max_speed[g] < RC(0) || !(m.infiltration[g] >= RC(0))) *P.odd = 1;
             P.peak_hi[L] = m.peak_hi[g];
             P.peak_lo[L] = m.peak_lo[g];
         }
