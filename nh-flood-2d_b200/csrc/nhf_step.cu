@@ -1248,6 +1248,7 @@ int nhf_initialize(nhf_handle *h)
     k_initialize<<<grid_for(n, 256), 256, 0, h->s>>>(h->dev);
     if (h->m.hang_cells > 0) k_hang_setup<<<grid_for(2 * h->m.hang_cells, 256), 256, 0, h->s>>>(h->dev);
 #ifndef NHF_REAL_DOUBLE
+    CK(h, cudaMemsetAsync(&h->ctl->dry_key, 0xff, sizeof(h->ctl->dry_key), h->s));   // kCflEmpty
     k_dry_key<<<148 * 4, 256, 0, h->s>>>(h->dev);
     if (h->resident) resident_enqueue_setup(h->dev, h->rb, h->s);
 #endif
