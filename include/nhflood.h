@@ -53,8 +53,10 @@ extern "C" {
 #define NHF_STEP_BAD_CFL 2
 #define NHF_STEP_BAD_DT 3
 #define NHF_STEP_OVERSHOOT 4
-/* Not a clock status: the blocks of a resident batch lost one another (a
- * wait ran out); the batch's results are void and so are later ones. */
+/* Not a clock status, in a batch's first trace row: the blocks of a resident
+ * batch lost one another (a wait ran out). The batch is void: its rows, and the
+ * state in the caller's arrays. Later batches of the handle, alone or in an
+ * ensemble, do nothing and say the same until nhf_initialize. */
 #define NHF_STEP_STALLED 5
 
 /* The physics type of the build. The step computes in F32 as the

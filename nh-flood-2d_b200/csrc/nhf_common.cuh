@@ -47,12 +47,12 @@ struct Ctl {
     real limit_value[5];
     int32_t limit_ids[3];
     uint32_t trace[NHF_MAX_BATCH * NHF_TRACE_COLS];
+    int32_t stalled;                  // resident form: a wait ran out (follows the trace: one copy reads both)
     unsigned long long cfl_min_bits;  // FP64 build: the CFL minimum's bits, then
     int32_t cfl_arg_min;              // the lowest side id that attains it
     int32_t grad_parity;              // tiled form: 1 when the last step's gradients are in the second buffer
     unsigned long long dry_key;       // the least CFL key of an all-dry state (initialize)
     uint32_t epoch, batches;          // resident form: steps and batches so far
-    int32_t stalled;                  // resident form: a wait ran out
     int32_t stepped;                  // 1 when the last slot's step ran (written by its commit only)
 };
 
@@ -79,6 +79,7 @@ struct ResidentArgs {
     TilePlan plan;
     int32_t max_don, max_hang, max_r1, max_owned;  // donor cells, hanging sides, ring-1 cells, owned sides of a tile
     int32_t max_per_face;       // sides of a face
+    int32_t spin_limit;         // reads of a word before a wait gives up
     uint32_t words[4];          // the batch's target and origin ticks
     // two buffers each, by the parity of the step
     unsigned long long *keys;         // [2][tiles] phase bit, CFL bits, side id
@@ -436,6 +437,15 @@ __device__ __forceinline__ void prepare_step(const Dev &d, Ctl *c, const real *d
     }
 }
 
+// A handle whose resident batch stalled runs no step until it is initialized: a
+// batch graph's begin has no target then, and its first row says so.
+__device__ __forceinline__ void begin_stalled(Ctl *c)
+{
+    c->next[0] = c->now[0]; c->next[1] = c->now[1];
+    c->done_blocks = 0;
+    c->trace[3] = NHF_STEP_STALLED;
+}
+
 // finish_step + StepClock.commit (solver_compact.py:384-391, clock.py:173-181)
 __device__ __forceinline__ void finish_step(Ctl *c)
 {
@@ -698,14 +708,15 @@ struct ResidentBuild {
     void *tables = nullptr, *memory = nullptr;  // owned (cudaFree on destroy)
     void *kernel = nullptr;
     int threads = 0, patterns = 0;
-    size_t shared_bytes = 0;
+    size_t shared_bytes = 0, words_bytes = 0;   // words_bytes: of `memory`, from its start
 };
 // Plan it when every tile of some size can be resident at once; 0 on success,
 // else nonzero with `why` set.
 int resident_build(const nhf_mesh &m, int terms, bool theta_one, cudaStream_t s, ResidentBuild *out, char *why,
                    size_t why_len);
-// Once the hanging gradients are laid out: the exchange flags.
-void resident_enqueue_setup(const Dev &d, const ResidentBuild &b, cudaStream_t s);
+// Once the hanging gradients are laid out: the exchange flags, and words and
+// counters as for a first batch (also after a stalled one).
+cudaError_t resident_enqueue_setup(const Dev &d, ResidentBuild &b, cudaStream_t s);
 // One batch towards words {target, origin}; the trace is in the control block.
 cudaError_t resident_enqueue_batch(const Dev &d, const ResidentBuild &b, const uint32_t words[4], cudaStream_t s);
 

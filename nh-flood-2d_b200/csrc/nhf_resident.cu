@@ -22,8 +22,12 @@
 // so no result travels back, while the other warps collect the outer rings and
 // reduce budget terms. Having everyone's key of step s also says that everyone
 // has read the words of step s - 1, so two buffers of words suffice. The grid
-// is launched cooperatively (all blocks resident at once); a wait gives up
-// after kSpinLimit reads, marks the batch stalled and the blocks leave.
+// is launched cooperatively (all blocks resident at once). A wait gives up after
+// kSpinLimit reads (NHF_RESIDENT_SPINS in the environment at nhf_initialize
+// sets another limit), its thread waits for nothing more and its block leaves;
+// the others' waits for that block run out in turn. The batch is void then, its
+// first trace row says NHF_STEP_STALLED, and so do later batches until
+// nhf_initialize.
 //
 // Measured, one batch of 32 steps end to end, against a launch per step:
 // 83 x 61 cells 646 to 271 us, 256 x 256 682 to 352, 421 x 307 numbered by
@@ -35,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -72,9 +77,9 @@ __device__ __forceinline__ u64 get_word(const u64 *p)
 __device__ __forceinline__ u64 value_word(float v, uint32_t step) { return ((u64)step << 32) | __float_as_uint(v); }
 
 // The value of step `step` at p, given a first read w of it.
-__device__ __forceinline__ float await_value(const u64 *p, u64 w, uint32_t step, bool &lost)
+__device__ __forceinline__ float await_value(const u64 *p, u64 w, uint32_t step, int limit, bool &lost)
 {
-    for (int spin = 0; (uint32_t)(w >> 32) != step && spin < kSpinLimit; ++spin) w = get_word(p);
+    for (int spin = 0; (uint32_t)(w >> 32) != step && spin < limit && !lost; ++spin) w = get_word(p);
     lost = lost || (uint32_t)(w >> 32) != step;
     return __uint_as_float((uint32_t)w);
 }
@@ -229,10 +234,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
     const int cbase = h2.y, sbase = h2.z;
     const int32_t *ext = P.ext_rel + h2.w, *srel = P.side_rel + h3.x;
 
-    if (c->stalled) {   // an earlier batch stalled: its words are out of step
-        if (blockIdx.x == 0 && tid == 0) c->trace[3] = NHF_STEP_STALLED;
-        return;
-    }
+    if (c->stalled) return;   // an earlier batch stalled: its words are out of step
 
     // ---- the tile, once per batch
     const int raining = c->raining;
@@ -727,7 +729,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
             u64 least = ~kPhase;
 #pragma unroll
             for (int k = 0; k < kMaxKeys; ++k) {
-                for (int spin = 0; (got[k] & kPhase) != phase && spin < kSpinLimit; ++spin)
+                for (int spin = 0; (got[k] & kPhase) != phase && spin < r.spin_limit && !lost; ++spin)
                     got[k] = get_word(keys + lane + 32 * k);
                 lost = lost || (got[k] & kPhase) != phase;
                 got[k] &= ~kPhase;
@@ -795,7 +797,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
                     if (to[k]) w[k] = get_word(p[k]);
 #pragma unroll
                 for (int k = 0; k < kAhead; ++k)
-                    if (to[k]) *to[k] = await_value(p[k], w[k], step, lost);
+                    if (to[k]) *to[k] = await_value(p[k], w[k], step, r.spin_limit, lost);
             }
             if (!kThetaOne) {   // a face of ring 2 towards ring 3: the discharge beyond it
                 const u64 *face_words = r.face_words + 4 * (size_t)(epoch & 1u) * m.e_num;
@@ -806,7 +808,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
                     if (a <= n_don && b <= n_don) continue;
                     const u64 *p = face_words + (a > n_don ? 4 * (size_t)(cbase + ext[a]) + (vertical ? 0 : 2)
                                                            : 4 * (size_t)(cbase + ext[b]) + (vertical ? 1 : 3));
-                    sh_nb[j] = await_value(p, get_word(p), step, lost);
+                    sh_nb[j] = await_value(p, get_word(p), step, r.spin_limit, lost);
                 }
             }
             if constexpr (kTwo) {
@@ -824,7 +826,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
 #pragma unroll
                     for (int o = 0; o < 5; ++o) { w[o] = get_word(p[o]); z[o] = m.bed[p[o] - depth_words]; }
 #pragma unroll
-                    for (int o = 0; o < 5; ++o) h[o] = await_value(p[o], w[o], step, lost);
+                    for (int o = 0; o < 5; ++o) h[o] = await_value(p[o], w[o], step, r.spin_limit, lost);
                     const real ha[2][2] = {{h[1], h[2]}, {h[3], h[4]}}, za[2][2] = {{z[1], z[2]}, {z[3], z[4]}};
                     e.value[k & 1] = hang_from(it, h[0], z[0], ha, za, d.min_h);
                 }
@@ -832,7 +834,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
         }
         epoch += 1;
         if (__syncthreads_or(lost)) {   // the batch is void: the host refuses its trace
-            if (tid == 0) { c->stalled = 1; c->trace[3] = NHF_STEP_STALLED; }
+            if (tid == 0) c->stalled = 1;
             return;
         }
     }
@@ -938,6 +940,12 @@ __global__ void k_resident_setup(const __grid_constant__ Dev d, const __grid_con
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < 8 * NHF_MAX_BATCH; i += blockDim.x)
             r.counts[i] = (i & 3) == 3 ? __float_as_uint(1.0f) : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the words are zero again
+        Ctl *c = d.ctl;
+        c->epoch = c->batches = 0u;
+        c->done_blocks = 0u;
+        c->stalled = 0;
+    }
 }
 
 template <int NT, int T>
@@ -1016,6 +1024,7 @@ int resident_build(const nhf_mesh &m, int terms, bool theta_one, cudaStream_t s,
             cudaFree(tb.device_memory);
             return no("no device memory for the resident form");
         }
+        r.spin_limit = kSpinLimit;
         r.keys = (unsigned long long *)(mem + o_key);
         r.depth_words = (unsigned long long *)(mem + o_dep);
         r.side_words = (unsigned long long *)(mem + o_side);
@@ -1024,6 +1033,7 @@ int resident_build(const nhf_mesh &m, int terms, bool theta_one, cudaStream_t s,
         r.need_cell = (int32_t *)(mem + o_nc);
         r.need_side = (uint8_t *)(mem + o_ns);
         out->args = r;
+        out->words_bytes = o_cnt;
         out->tables = tb.device_memory;
         out->memory = mem;
         out->kernel = kernel;
@@ -1035,9 +1045,14 @@ int resident_build(const nhf_mesh &m, int terms, bool theta_one, cudaStream_t s,
     return no("tiles do not fit the GPU at once");
 }
 
-void resident_enqueue_setup(const Dev &d, const ResidentBuild &b, cudaStream_t s)
+cudaError_t resident_enqueue_setup(const Dev &d, ResidentBuild &b, cudaStream_t s)
 {
+    const char *spins = getenv("NHF_RESIDENT_SPINS");
+    b.args.spin_limit = spins && atoi(spins) >= 0 ? atoi(spins) : kSpinLimit;
+    const cudaError_t e = cudaMemsetAsync(b.memory, 0, b.words_bytes, s);
+    if (e != cudaSuccess) return e;
     k_resident_setup<<<b.args.plan.n_tiles, 256, 0, s>>>(d, b.args);
+    return cudaGetLastError();
 }
 
 cudaError_t resident_enqueue_batch(const Dev &d, const ResidentBuild &b, const uint32_t words[4], cudaStream_t s)

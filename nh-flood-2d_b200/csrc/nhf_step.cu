@@ -91,6 +91,7 @@ __global__ void k_begin(Dev d, uint32_t next_hi, uint32_t next_lo, uint32_t orig
     }
     for (int i = t; i < NHF_MAX_BATCH * NHF_TRACE_COLS; i += blockDim.x) c->trace[i] = 0u;
     __syncthreads();
+    if (t == 0 && c->stalled) begin_stalled(c);
     if (prepare_first && t == 0) prepare_step(d, c, d.m.depth, d.m.q);
 }
 
@@ -1155,7 +1156,8 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     h->ctl = (Ctl *)(base + o_ctl);
     h->d_begin = (uint32_t *)(base + o_begin);
     CKC(cudaMallocHost(&h->h_begin, 4 * sizeof(uint32_t)));
-    CKC(cudaMallocHost(&h->h_trace, sizeof(uint32_t) * NHF_TRACE_COLS * NHF_MAX_BATCH));
+    CKC(cudaMallocHost(&h->h_trace, sizeof(Ctl::trace) + sizeof(Ctl::stalled)));
+    memset(h->h_trace, 0, sizeof(Ctl::trace) + sizeof(Ctl::stalled));
     CKC(cudaMallocHost(&h->h_small, sizeof(real) * (2 * bb + nr + 64)));
     CKC(cudaMallocHost(&h->h_acc, sizeof(double) * 2 * (size_t)blocks * T + 16));
     Dev &d = h->dev;
@@ -1250,7 +1252,7 @@ int nhf_initialize(nhf_handle *h)
 #ifndef NHF_REAL_DOUBLE
     CK(h, cudaMemsetAsync(&h->ctl->dry_key, 0xff, sizeof(h->ctl->dry_key), h->s));   // kCflEmpty
     k_dry_key<<<148 * 4, 256, 0, h->s>>>(h->dev);
-    if (h->resident) resident_enqueue_setup(h->dev, h->rb, h->s);
+    if (h->resident) CK(h, resident_enqueue_setup(h->dev, h->rb, h->s));
 #endif
     return leave(h);
 }
@@ -1347,7 +1349,8 @@ int nhf_run_batch_async(nhf_handle *h, const uint32_t target[2], const uint32_t 
 #ifndef NHF_REAL_DOUBLE
     if (h->resident) {
         CK(h, resident_enqueue_batch(h->dev, h->rb, w, h->s));
-        CK(h, cudaMemcpyAsync(h->h_trace, h->ctl->trace, sizeof(uint32_t) * NHF_TRACE_COLS * h->p.batch_size,
+        static_assert(offsetof(Ctl, stalled) == offsetof(Ctl, trace) + sizeof(Ctl::trace), "one copy for both");
+        CK(h, cudaMemcpyAsync(h->h_trace, h->ctl->trace, sizeof(Ctl::trace) + sizeof(Ctl::stalled),
                               cudaMemcpyDeviceToHost, h->s));
         return leave(h);
     }
@@ -1369,6 +1372,8 @@ int nhf_read_trace(nhf_handle *h, uint32_t *trace)
     if (!h || !trace) return NHF_EINVAL;
     CK(h, cudaStreamSynchronize(h->s));
     memcpy(trace, h->h_trace, sizeof(uint32_t) * NHF_TRACE_COLS * h->p.batch_size);
+    // (written by resident batches only)
+    if (h->h_trace[NHF_MAX_BATCH * NHF_TRACE_COLS]) trace[3] = NHF_STEP_STALLED;
     return NHF_OK;
 }
 

@@ -1320,6 +1320,7 @@ __global__ void k_ens_begin(const Dev *devs, const uint32_t *words)
     }
     for (int i = t; i < NHF_MAX_BATCH * NHF_TRACE_COLS; i += blockDim.x) c->trace[i] = 0u;
     __syncthreads();
+    if (t == 0 && c->stalled) begin_stalled(c);
     if (t == 0) prepare_step(d, c, d.m.depth, d.m.q);
 }
 

@@ -15,6 +15,7 @@ import numpy as np
 TICKS_PER_SECOND = 1 << 40
 MAX_TICKS = (1 << 64) - 1
 DONE, COMPLETED, BAD_CFL, BAD_DT, OVERSHOOT = 0, 1, 2, 3, 4
+STALLED = 5  # not a clock status: a resident batch is void (NHF_STEP_STALLED)
 
 
 def seconds_to_ticks(seconds: float) -> int:
@@ -80,6 +81,9 @@ class HostClock:
         n = int(stops[0]) if len(stops) else len(rows)
         if n:
             self.now_ticks = ticks_of(rows[n - 1][1], rows[n - 1][2])
+        if len(rows) and int(status[0]) == STALLED:
+            raise RuntimeError('The blocks of a resident batch lost one another (trace status 5): the batch is void; '
+                               'initialize the engine and set its state again')
         # an unknown status is refused after the completed rows before it
         # have advanced the clock, and the batch stays pending
         if n < len(rows) and int(status[n]) not in (BAD_CFL, BAD_DT, OVERSHOOT, DONE):

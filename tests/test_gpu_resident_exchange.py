@@ -1,9 +1,10 @@
 """What the blocks of a resident batch tell one another beyond the state: the
-limiting side's snapshot, whose owner changes from step to step."""
+limiting side's snapshot, whose owner changes from step to step; and a batch
+whose blocks lose one another (a wait that may not wait runs out)."""
 import numpy as np
 import pytest
 
-from test_gpu_resident import assert_same, engine
+from test_gpu_resident import assert_same, engine, grid, quadtree
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +48,49 @@ def test_snapshot_of_changing_owners(cuda_available, batch):
         assert len(owners[0]) > 3    # tiles that held the limit during the first batch
     for r in (a, b, one):
         r.close()
+
+
+STALLED = 5
+
+
+@pytest.mark.parametrize('make', [lambda: grid(83, 61), lambda: grid(70, 33, rows=True, theta=0.8), lambda: quadtree(1200)],
+                         ids=['grid', 'theta', 'quadtree'])
+def test_a_stalled_batch_is_reported_until_initialize(cuda_available, monkeypatch, make):
+    import time
+    from nhflood.native import CudaEnsemble
+    from nhflood.plain import PlainRun
+    w = make()
+    arrays = w.step_arrays()
+    monkeypatch.setenv('NHF_RESIDENT_SPINS', '0')    # read by nhf_initialize
+    run = PlainRun(w, engine('auto'), arrays=arrays)
+    words = run.begin()
+    started = time.perf_counter()
+    rows = run.engine.run_batch(*words)
+    assert time.perf_counter() - started < 5
+    assert rows[0, 3] == STALLED
+    with pytest.raises(RuntimeError, match='lost one another'):
+        run.finish(rows)
+    assert run.clock.pending and run.clock.now_ticks == 0
+    # later batches of the handle say the same, resident, as member graphs and in one launch
+    assert run.engine.run_batch(*words)[0, 3] == STALLED
+    other = PlainRun(w, engine('steps'), arrays=arrays)
+    for blocks in (-2, -1):
+        ens = CudaEnsemble([run.engine, other.engine], blocks)
+        theirs = other.begin()
+        traces = ens.run_batch(*(np.array(x, np.uint32) for x in zip(words, theirs)))
+        assert traces[0][0, 3] == STALLED and (traces[0][1:, 3] == 0).all()
+        other.finish(traces[1])
+        ens.close()
+    other.close()
+    # initialized again with the usual limit: a run like any other
+    monkeypatch.delenv('NHF_RESIDENT_SPINS')
+    run.engine.budget_flush()
+    run.engine.reset_limits()
+    for name in ('q', 'rain_time'):
+        run.engine.set(name, np.zeros_like(run.engine.get(name)))
+    again, fresh = PlainRun(w, lambda a, p: run.engine, arrays=arrays), PlainRun(w, engine('auto'), arrays=arrays)
+    for _ in range(3):
+        again.advance(), fresh.advance()
+    assert again.steps == fresh.steps > 32
+    assert_same(again, fresh)
+    again.close(), fresh.close()
