@@ -21,6 +21,7 @@ else was resident: alone and in the mix are bit-identical.
 """
 from __future__ import annotations
 
+import os
 import time
 from collections import deque
 from concurrent.futures import ThreadPoolExecutor
@@ -32,32 +33,68 @@ from .ensemble import MEMBER_GRAPHS, plain_factory, tiled_factory
 from .plain import PlainRun
 
 
-def device_bytes_estimate(arrays) -> int:
+LATTICE_CELLS = 1 << 18  # uniform grids of at least so many cells run on the lattice (nhf_create, path 4)
+
+
+def tiled_bytes(e: int, s: int) -> int:
+    """Second state buffers and the tile plan of the fused step."""
+    return 4 * (3 * e + s) + 28 * e + 64 * 1024
+
+
+def lattice_bytes(x, y, cell: float, e: int, s: int, terms: int, horton: bool, rain_cells: bool) -> int:
+    """What the lattice form allocates (lattice_build in csrc/nhf_lattice.cu):
+    per lattice point, cell, side, budget block and warp, for chunks of the
+    tallest rows it takes."""
+    nx, ny = (int(round((float(v[1:].max()) - float(v[1:].min())) / cell)) + 1 for v in (x, y))
+    rows = max(16, int(os.environ.get('NHF_LATTICE_ROWS') or 0))
+    strips = (nx + 28) // 28
+    height = ny + 1 + rows                        # whole chunks over cell rows 0..ny
+    points = (strips * 28 + 4) * (height + 5)
+    per_point = 12 + 1 + 24 + 12 + 2 + 16 + 8 + (4 if rain_cells else 0) + (12 if horton else 0)
+    warps = strips * (height // 2 + 1)            # chunks of two rows at least, unless one is asked for
+    if os.environ.get('NHF_LATTICE_ROWS') == '1':
+        warps *= 2
+    return per_point * points + 4 * (e + s) + 4 * terms * e + 5 * (e // 256 + 1) + 25 * warps + \
+        24 * strips * height + 40 * 256
+
+
+def device_bytes_estimate(arrays, lattice: bool = True) -> int:
     """Device bytes one resident solve holds: its uploaded inputs, the
     state (bed, depth, q, rain_time, infiltration, extrema, u, v, peak
-    words), and the library scratch of the fused step (centre distances,
-    donor factors, face fluxes, second state buffers, budget partials, tile
-    plan)."""
+    words), the library's scratch (centre distances, donor factors, face
+    fluxes, budget partials, hanging-edge gradients) and what its step form
+    adds: second state buffers and tile plan, or the lattice's arrays on a
+    uniform grid that runs on it (``lattice``: the engine may choose it, as in
+    the member graphs)."""
     e, s = arrays.e_num, arrays.s_num
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 3 * e + s) + 16 * ((e + 255) // 256) * arrays.terms + 136 * arrays.hang_cells
-    plan = 28 * e + 64 * 1024
-    return int(arrays.nbytes() + state + scratch + plan + (1 << 20))
+    scratch = 4 * (s + e + 4 * e) + 16 * ((e + 255) // 256) * arrays.terms + 136 * arrays.hang_cells
+    form = tiled_bytes(e, s)
+    if (lattice and e > LATTICE_CELLS and not arrays.hang_cells and arrays.open_face is None and arrays.b_num <= 4
+            and len(arrays.isl_data) == 4 * (e - 1) and (arrays.width[1:] == arrays.width[1]).all()):
+        horton = any(v[1:].any() for v in (arrays.f0, arrays.fc, arrays.k))
+        form = max(form, lattice_bytes(arrays.x, arrays.y, float(arrays.width[1]), e, s, arrays.terms, horton,
+                                       bool(arrays.rain_index[1:].any())))
+    return int(arrays.nbytes() + state + scratch + form + (1 << 20))
 
 
-def device_bytes_bound(workload) -> int:
+def device_bytes_bound(workload, lattice: bool = True) -> int:
     """An upper bound of device_bytes_estimate from the mesh sizes alone
     (before the step arrays are built): hanging-edge tables counted as if
     every side had one, gradient cells as all the cells at faces of several
-    sides."""
+    sides; a lattice with soil and rain of its own in every cell."""
     m = workload.mesh
     e, s, isl = m.e_num, m.s_num, len(m.isl_data)
     hanging = min(e, 2 * int(m.counts[m.counts > 1].sum()))
-    terms = 4 + 6 * len(workload.forcing.boundaries)
+    boundaries = len(workload.forcing.boundaries)
+    terms = 4 + 6 * boundaries
     inputs = 4 * (12 * e + 8 * e + isl) + 21 * s + 16 * e + 44 * s
     state = 4 * (10 * e + s)
-    scratch = 4 * (s + e + 4 * e + 3 * e + s) + 16 * ((e + 255) // 256) * terms + 136 * hanging
-    return int(inputs + state + scratch + 28 * e + 64 * 1024 + (1 << 20))
+    scratch = 4 * (s + e + 4 * e) + 16 * ((e + 255) // 256) * terms + 136 * hanging
+    form = tiled_bytes(e, s)
+    if lattice and e > LATTICE_CELLS and not hanging and workload.sita == 1.0 and boundaries <= 4 and isl == 4 * (e - 1):
+        form = max(form, lattice_bytes(m.x, m.y, float(m.side_length[1:].min()), e, s, terms, True, True))
+    return int(inputs + state + scratch + form + (1 << 20))
 
 
 @dataclass
@@ -193,7 +230,7 @@ class FloodServer:
         started = 0
         while self.waiting:
             req = self.waiting[0]
-            need = device_bytes_bound(req.resolve())
+            need = device_bytes_bound(req.resolve(), self.grid_blocks == MEMBER_GRAPHS)
             if need > self.budget:
                 raise ValueError(f'request {req.id} needs {need} B, more than the whole budget')
             if self.used + need > self.budget:
@@ -226,7 +263,7 @@ class FloodServer:
         while self.building and (self.building[0][1].done() or wait):
             req, future, bound = self.building.popleft()
             run = future.result()
-            need = device_bytes_estimate(run.arrays)
+            need = device_bytes_estimate(run.arrays, self.grid_blocks == MEMBER_GRAPHS)
             self.used += need - bound
             self.active.append((req, run, need, self.now()))
             self.dirty = True
@@ -330,7 +367,7 @@ def serve_sequential(requests, *, tile: int = 256, batch_size: int = 32, device:
         while not run.done:
             run.advance()
         out.append(Completed(req.id, req.arrival, started, clock() - t0, run.w.cells, run.steps,
-                             device_bytes_estimate(run.arrays), run.engine.get('depth'), run.engine.get('max_depth')))
+                             device_bytes_estimate(run.arrays, False), run.engine.get('depth'), run.engine.get('max_depth')))
         run.close()
     return out
 
