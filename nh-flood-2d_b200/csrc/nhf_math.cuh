@@ -125,17 +125,18 @@ __device__ __forceinline__ float approx_sqrt(float x)
     return r;
 }
 
-// Whether an FP64 value lies so near the midpoint of two F32 neighbours (4096
-// FP64 units, at least 2^-41 of the value) that a relative error of 2^-41
-// could change its rounding to F32.
+// Whether an FP64 value lies so near the midpoint of two F32 neighbours that a
+// relative error of 2^-40 (kOpenUnits FP64 units, at least) could change its
+// rounding to F32.
+constexpr uint32_t kOpenUnits = 8192;
 __device__ __forceinline__ bool rounding_open(double v)
 {
     const uint32_t below = (uint32_t)__double_as_longlong(v) & 0x1fffffffu;  // the 29 bits F32 drops
-    return below - (0x10000000u - 4096u) < 8192u;
+    return below - (0x10000000u - kOpenUnits) < 2 * kOpenUnits;
 }
 
 // The full evaluations behind the rounding test, out of line: about one in
-// 2^16 arguments gets here.
+// 2^15 arguments gets here.
 static __device__ __noinline__ float pow73_full(float x) { return pow_f32(x, 0x1.2aaaaap+1f); }
 static __device__ __noinline__ float exp_full(float a) { return exp_f32(a); }
 
@@ -144,8 +145,9 @@ static __device__ __noinline__ float exp_full(float a) { return exp_f32(a); }
 // x^y = x^3 (x^(-1/3))^2 x^(-c). x^(-1/3) is an F32 estimate s (relative
 // error below 2^-18) corrected by the binomial series of (1 - t)^(-1/3) at
 // t = 1 - x s^3, whose third term is under 2^-50; x^(-c) is 1 + w + w^2 / 2 at
-// w = -c ln x, |w| < 2e-6, in F32 (error under 2^-43). 11 FP64 operations
-// instead of about 85, and a shorter chain, which is what a small step's
+// w = -c ln x, |w| < 2^-19.7, in F32: the logarithm's 2^-22 and three roundings
+// make at most 2^-40.9 of the value, at 2^20, and less than that at smaller x.
+// 11 FP64 operations instead of about 85, and a shorter chain, which is what a small step's
 // momentum waits for. Measured together with horton_exp, cfl_above and
 // speed_not_above (nhf_common.cuh), 32 steps: 256 x 256 cells 732 to 682 us,
 // 2048 x 1531 cells with Horton soil 9.34 to 7.95 ms, quadtree of 1.36 M cells
@@ -166,7 +168,7 @@ __device__ __forceinline__ float friction_pow(float x)
 
 // exp(a) of the Horton capacity, a <= 0: the value of exp_f32(a). One-step
 // reduction by ln 2 (|a| < 80: error under 2^-46) and the Taylor series to
-// degree 10 (remainder under 2^-41.9 for |r| <= ln2 / 2) with fused
+// degree 10 (remainder under 2^-41.5 of the value for |r| <= ln2 / 2) with fused
 // multiply-adds: 14 FP64 operations instead of about 40.
 __device__ __forceinline__ float horton_exp(float a)
 {
