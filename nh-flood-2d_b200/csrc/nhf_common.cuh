@@ -151,7 +151,7 @@ struct GateDev {
 
 struct Dev {
     nhf_mesh m;
-    real g, neg_g, afa, sita, half_rest, seven_thirds, min_h;
+    real g, neg_g, afa, sita, half_rest, min_h;
     float min_dt;
     int32_t terms, blocks, batch_size, theta_one;
     Ctl *ctl;

@@ -91,7 +91,7 @@ __device__ __forceinline__ real lattice_momentum(const Dev &d, real dt, real za,
         const real xdq = (exterior ? slope / d.sdc[at(side_ids, off)] : over(slope, sdc, inverse)) *
                          rmaxc(xwh, RC(0)) * dt;
         real ratio = RC(0);
-        if (xq != RC(0)) ratio = xq / pow_real(rmaxc(xwh, RC(0.00001)), d.seven_thirds);
+        if (xq != RC(0)) ratio = xq / friction_pow_real(rmaxc(xwh, RC(0.00001)));
         const real xf = RC(1) + d.g * dt * (n * n) * fabs(ratio);
         const real nb = RC(0) + RC(0);
         new_q = (d.sita * xq + d.half_rest * nb + xdq) / xf;

@@ -190,19 +190,19 @@ __device__ __forceinline__ float horton_exp(float a)
     return (float)p;
 }
 
-// The friction power and the Horton exponential in the build's physics type:
-// rounded once to F32, or in the FP64 build kept in double.
+// The friction power x^(7/3) and the Horton exponential in the build's physics
+// type: rounded once to F32 (the power with the exponent f32(7/3)), or in the FP64
+// build kept in double.
 #ifdef NHF_REAL_DOUBLE
-__device__ __forceinline__ double pow_real(double x, double y)
+__device__ __forceinline__ double friction_pow_real(double x)
 {
     if (x != x) return x;
     if (x == 0.0) return 0.0;
-    return exp_f64(y * ln_f64(x));
+    return exp_f64(7.0 / 3.0 * ln_f64(x));
 }
 __device__ __forceinline__ double exp_real(double a) { return exp_f64(a); }
 #else
-// (the F32 step's exponent is f32(7/3) throughout)
-__device__ __forceinline__ float pow_real(float x, float) { return friction_pow(x); }
+__device__ __forceinline__ float friction_pow_real(float x) { return friction_pow(x); }
 __device__ __forceinline__ float exp_real(float a) { return horton_exp(a); }
 #endif
 

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ Dev 
                 if (kTwo && hanging && da > d.min_h && db > d.min_h) difference = difference - part0 - part1;
                 const float xdq = (d.neg_g * difference / sh_dx[j]) * maxf(xwh, 0.0f) * dt;
                 float ratio = 0.0f;
-                if (xq != 0.0f) ratio = xq / pow_real(maxf(xwh, 0.00001f), d.seven_thirds);
+                if (xq != 0.0f) ratio = xq / friction_pow_real(maxf(xwh, 0.00001f));
                 const float xf = 1.0f + d.g * dt * (n * n) * fabsf(ratio);
                 const float nb = kThetaOne ? 0.0f + 0.0f : sh_nb[j];
                 new_q = (d.sita * xq + d.half_rest * nb + xdq) / xf;

@@ -199,7 +199,7 @@ __global__ void k_sides(Dev d)
     real ratio = RC(0.0);
     // xq / p with p = max(wh, 1e-5) ** f32(7/3) > 0: a zero discharge gives a
     // zero ratio without evaluating the power (identical bits).
-    if (xq != RC(0.0)) ratio = xq / nhf::pow_real(rmax(xwh, RC(0.00001)), d.seven_thirds);
+    if (xq != RC(0.0)) ratio = xq / nhf::friction_pow_real(rmax(xwh, RC(0.00001)));
     real xf = RC(1.0) + d.g * dt * (n * n) * fabs(ratio);
     int dl = so == 2 ? 0 : 2, dr = so == 2 ? 1 : 3;
     real nb;
@@ -1167,7 +1167,6 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
     d.afa = params->afa;
     d.sita = params->sita;
     d.half_rest = (real)((1.0 - (double)params->sita) / 2.0);
-    d.seven_thirds = (real)(7.0 / 3.0);
     d.min_h = params->min_h;
     d.min_dt = params->min_dt;
     d.terms = T;

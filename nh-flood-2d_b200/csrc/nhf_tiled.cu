@@ -367,7 +367,7 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
             }
             float xdq = (d.neg_g * difference / dx) * rmaxc(xwh, 0.0f) * dt;
             float ratio = 0.0f;
-            if (xq != 0.0f) ratio = xq / pow_real(rmaxc(xwh, 0.00001f), d.seven_thirds);
+            if (xq != 0.0f) ratio = xq / friction_pow_real(rmaxc(xwh, 0.00001f));
             float xf = 1.0f + d.g * dt * (n * n) * fabsf(ratio);
             float nb;
             if (kThetaOne) {
