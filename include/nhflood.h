@@ -116,17 +116,21 @@ typedef struct nhf_params {
                            cooperative launch) when one tile per SM covers
                            the mesh, else the lattice form on a uniform grid
                            it covers of at least 2^18 cells (2^20 with
-                           cfl_mode 2), else the fused tiled step when the mesh allows it, else
-                           multi-pass; 4: the same without the resident form
-                           (members of an ensemble, which run beside others); 1: always the multi-pass step;
+                           cfl_mode 2), else the fused tiled step when the
+                           mesh allows it, else multi-pass; 4: the same
+                           without the resident form (members of an ensemble,
+                           which run beside others); 1: always the multi-pass
+                           step;
                            2: the lattice form when the mesh allows it, else
                            multi-pass; 3: the fused tiled step (tile size by
                            mesh size) when the mesh allows it, else multi-pass;
                            256, 512 or 1024: fused tiled step with that tile
                            size when the mesh allows it, else multi-pass */
     int32_t cfl_mode;   /* fused step only. 0: the next step's CFL candidate
-                           in the step itself on meshes of less than two
-                           waves of tiles, else a separate pass after it;
+                           in the step itself on meshes without hanging edges
+                           of less than 1480 tiles of 256 cells (592 larger
+                           ones), else that of the sides between tiles in a
+                           pass after it;
                            1: always in the step; 2: always a separate pass
                            (ensemble members, whose launches span all
                            members) */

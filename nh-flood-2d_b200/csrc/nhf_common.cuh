@@ -677,8 +677,9 @@ struct TiledBuild {
 // once). Returns 0 on success; a nonzero value with `why` set when the mesh
 // does not fit the tiled form (the caller then keeps the multi-pass form).
 // tile_request: 0 picks the tile size by mesh size; 256, 512 or 1024 asks
-// for that size only. cfl_mode: 0 separate CFL pass from two waves of tiles
-// on, 1 CFL always in the step, 2 always a separate pass. With `resident` the
+// for that size only. cfl_mode: 0 separate CFL pass from 1480 tiles of 256 cells
+// (592 larger ones) on and wherever edges hang, 1 CFL always in the step, 2 always a
+// separate pass. With `resident` the
 // plan serves the resident form: its largest lists are reported there and the
 // caller checks shared memory.
 int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, size_t why_len,

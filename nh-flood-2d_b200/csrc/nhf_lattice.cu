@@ -434,9 +434,10 @@ __device__ __forceinline__ void lattice_rows(const Dev &d, const int strip, cons
 // buffer 0 and a step that does nothing is followed by none that does), so the
 // array bases are kernel parameters.
 //
-// Bound by instruction issue and memory latency (57 % of cycles issue with 28
-// of 64 warps, DRAM at 20 %): 32 warp instructions per cell, 37 before the
-// inner path without liveness, boundaries and exterior sides (lattice_rows),
+// Bound by instruction issue and memory latency (2048 x 1531 with Horton soil,
+// 170 us: 59 % of active cycles issue with 21 of 64 warps, 24 by its 80 registers
+// with 44 bytes of spills; DRAM at 20 %): 31 warp instructions per cell, 37
+// before the inner path without liveness, boundaries and exterior sides (lattice_rows),
 // 32-bit offsets on constant bases, rain rates instead of pixels and the rows
 // that stay dry skipped. With the close pass that reduces a budget block per
 // warp instead of per thread block (48 to 21 us at 2048 x 1531 with Horton

@@ -1079,11 +1079,18 @@ int nhf_create(const nhf_mesh *mesh, const nhf_params *params, void *stream, nhf
         }
     }
     // Lattice form when the mesh is a uniform grid it covers (params->path 2, or
-    // a grid of at least 2^18 cells that does not run resident: 600 x 600 cells
-    // 1357 us per 32 steps against 1603 on tiles, 1003 x 741 2047 against 2806
-    // (numbered by rows 2054 against 4580), 421 x 307 1037 against 983). A caller
-    // that places the CFL in a pass of its own keeps the tiles up to 2^20 cells,
-    // where a gate controller can be attached to them.
+    // a grid of at least 2^18 cells that does not run resident). Resident batches
+    // are twice as fast where they fit, up to about 0.3 M cells (us per 32 steps,
+    // wet hills with Horton soil, resident, lattice, tiles: 512 x 512 722, 1456,
+    // 1148; 544 x 544 727, 1491, 1226). What does not fit: numbered by rows the
+    // lattice wins at once (544 x 544 1445 against 1606 multi-pass, 800 x 800 1914
+    // against 3852 on tiles); numbered by compact tiles it wins from about 0.6 M
+    // cells on (800 x 800 2021 against 2044, 1000 x 1000 2958 against 3123), is even
+    // at 600 x 600 (1402 against 1480) and loses below and between (550 x 550 1488
+    // against 1312, 700 x 700 1957 against 1855), where half dry grids gain
+    // (600 x 600 1357 against 1603). A caller that places the CFL in a pass of its
+    // own keeps the tiles up to 2^20 cells, where a gate controller can be attached
+    // to them.
     const int lattice_from = params->cfl_mode == 2 ? 1 << 20 : 1 << 18;
     if (!h->resident && (params->path == 2 || (any_form && mesh->e_num - 1 >= lattice_from))) {
         Dev probe{};

@@ -713,9 +713,9 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
     // owned side in the fused-CFL form; in the split form of those whose two
     // cells are the tile's (the edge pass takes the others, and those of gate
     // cells, whose beds move first), unless a full CFL pass follows (ensemble
-    // launches). Starting
-    // from the minimum of the blocks that are done spares 4 % of the instructions
-    // but its hot word costs more (1.36 M cells: 4538 to 4661 us per 32 steps).
+    // launches). Starting from the minimum of the blocks that are done spares 4 %
+    // of the instructions but its hot word costs more (1.36 M cells: 4538 to 4661
+    // us per 32 steps).
     const bool split = P.split != 0;
     const int last_cell = !split ? tl.n_ext : kHang == 2 ? 0 : tl.n_r0;
     unsigned long long best = kCflEmpty;
@@ -775,9 +775,9 @@ __device__ __forceinline__ void step_tile(const Dev &d, const int t_index, const
 
 // CFL pass (solver_compact.py:617-641), block `block` of `blocks`, over sides
 // [first, end) with stride (or, kEdges, over the plan's sides between tiles), on
-// the current (just updated) state; each block adds its minimum packed key (cfl bits, side id) and the
-// last of `blocks` blocks sets ndt / cfl_arg (the lowest side id attains the
-// minimum) and prepares the next step (solver_compact.py:364-382).
+// the current (just updated) state; each block adds its minimum packed key (cfl
+// bits, side id) and the last one sets ndt / cfl_arg (the lowest side id attains
+// the minimum) and prepares the next step (solver_compact.py:364-382).
 template <bool kEdges = false>
 __device__ __forceinline__ void cfl_pass(const Dev &d, unsigned block, unsigned blocks, int first, int end, int stride,
                                          const GateDev *gd = nullptr)
@@ -1426,7 +1426,7 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
     size_t smem = 0;
     // Small meshes take small tiles so that every SM gets work.
     // Multi-resolution meshes (irregular halos, more work per cell) run best
-    // with 256-cell tiles and five blocks per SM; on uniform meshes large
+    // with 256-cell tiles and six blocks per SM; on uniform meshes large
     // tiles amortise the halo.
     std::vector<int> sizes = {1024, 512, 256};
     if (m.e_num < 148 * 2 * 1024 || m.hang_cells > 0) sizes = {256, 512, 1024};
@@ -1460,8 +1460,8 @@ int tiled_build(const nhf_mesh &m, cudaStream_t s, TiledBuild *out, char *why, s
         max_ext = (max_ext + 3) & ~3;   // every array of a tile starts on 16 bytes
         max_sides = (max_sides + 3) & ~3;
         // centre distance and Manning n are staged with the tile where that
-        // costs no resident block (members of 0.1 to 0.2 M cells with four
-        // blocks per SM instead of five ran 5 % slower)
+        // costs no resident block (measured at a limit of five: members of 0.1 to
+        // 0.2 M cells with four blocks per SM ran 5 % slower)
         const size_t lean = (size_t)max_ext * 28 + (size_t)max_sides * 16 + (size_t)((max_faces + 7) & ~7) * 2 + 16;
         auto resident_blocks = [&](size_t bytes) {
             return std::min(T == 256 ? kMinBlocks<256> : kMinBlocks<512>, (int)(228 * 1024 / (bytes + 1024 + 256)));

@@ -28,15 +28,16 @@ class StepParams:
     batch_size: int = 32
     g: float = float(G)
     min_dt: float = float(np.float32(MIN_DT))
-    # 'auto': the lattice form on large uniform grids, the resident form on
-    # meshes that fit the GPU at once, else the fused tiled step when the mesh
+    # 'auto': the resident form on meshes that fit the GPU at once, else the
+    # lattice form on large uniform grids, else the fused tiled step when the mesh
     # allows it, else multi-pass; 'steps': the same without the resident form
     # (ensemble members); 'lattice', 'tiled', 'tile256' /
     # 'tile512' / 'tile1024', 'multipass' ask for one form
     path: str = 'auto'
     # fused step: where the next step's CFL candidate is computed. 'auto': in
-    # the step on meshes of less than two waves of tiles, else in a separate
-    # pass; 'fused': always in the step; 'pass': always a separate pass
+    # the step on meshes without hanging edges of less than 1480 tiles of 256
+    # cells (592 larger ones), else in a separate pass; 'fused': always in the
+    # step; 'pass': always a separate pass
     cfl: str = 'auto'
 
 
